@@ -136,7 +136,6 @@ __device__ __forceinline__ void topn_insert(TopN<N>& t, float d, int idx) {
     }
   }
 }
-__device__ __forceinline__ void top5_insert(Top5& t, float d, int idx) { topn_insert<kJ>(t, d, idx); }
 
 __device__ __forceinline__ float knn_dist(float q0, float q1, float q2, float r0, float r1,
                                           float r2, const float* s) {
@@ -162,65 +161,6 @@ __device__ __forceinline__ int cell_coord(float y, float lo, float inv_h, int di
   return c;
 }
 
-// Exact grid search: rings of cells at growing Chebyshev distance r around the query's
-// cell; stop after ring r once the fifth distance is strictly below the squared lower
-// bound (r*h + delta - eps)^2 of every unvisited cell.  eps absorbs float rounding of
-// the scaled coordinates and of the distance itself.  Refs outside the box sit in the
-// boundary cells, which keeps the bound valid for queries inside the box.
-template <int N>
-__device__ void knn_grid_search(float q0, float q1, float q2, const float* s, const GridGeom& g,
-                                const int32_t* __restrict__ cstart, const float4* __restrict__ refs,
-                                TopN<N>& t) {
-  const float y[3] = {q0 * s[0], q1 * s[1], q2 * s[2]};
-  int c[3];
-  float delta = kInfF;
-#pragma unroll
-  for (int a = 0; a < 3; a++) {
-    c[a] = cell_coord(y[a], g.lo[a], g.inv_h, g.dims[a]);
-    float f0 = y[a] - (g.lo[a] + c[a] * g.h);
-    float f1 = (g.lo[a] + (c[a] + 1) * g.h) - y[a];
-    delta = fminf(delta, fminf(f0, f1));
-  }
-  delta = fmaxf(delta, 0.0f);
-  const int maxr = max(g.dims[0], max(g.dims[1], g.dims[2]));
-  for (int r = 0; r <= maxr; ++r) {
-    const int z0 = max(c[2] - r, 0), z1 = min(c[2] + r, g.dims[2] - 1);
-    const int y0 = max(c[1] - r, 0), y1 = min(c[1] + r, g.dims[1] - 1);
-    for (int z = z0; z <= z1; ++z) {
-      const bool zedge = (z == c[2] - r) || (z == c[2] + r);
-      for (int yy = y0; yy <= y1; ++yy) {
-        const bool edge = zedge || (yy == c[1] - r) || (yy == c[1] + r);
-        const int row = (z * g.dims[1] + yy) * g.dims[0];
-        int xa, xb, step;
-        if (edge) {
-          xa = max(c[0] - r, 0);
-          xb = min(c[0] + r, g.dims[0] - 1);
-          step = 1;
-        } else {
-          xa = c[0] - r;
-          xb = c[0] + r;
-          step = 2 * r;
-        }
-        for (int x = xa; x <= xb; x += step) {
-          if (x < 0 || x >= g.dims[0]) continue;
-          const int cell = row + x;
-          const int b = cstart[cell], e = cstart[cell + 1];
-          for (int k = b; k < e; ++k) {
-            const float4 rr = refs[k];
-            topn_insert<N>(t, knn_dist(q0, q1, q2, rr.x, rr.y, rr.z, s), __float_as_int(rr.w));
-          }
-        }
-      }
-    }
-    const float lb = r * g.h + delta;
-    const float eps = 4e-3f + 1e-6f * lb;
-    if (lb > eps) {
-      const float bound = (lb - eps) * (lb - eps);
-      if (t.d[N - 1] < bound) break;
-    }
-  }
-}
-
 __device__ __forceinline__ FrameDesc load_desc(const DevPlan& P, int f) { return P.frames[f]; }
 
 }  // namespace
@@ -228,7 +168,8 @@ __device__ __forceinline__ FrameDesc load_desc(const DevPlan& P, int f) { return
 
 // Grid geometry over the bounding box [lo, hi] (scaled space): cubic cells of side h,
 // about one reference per cell, at most budget-1 cells in total.
-__device__ void set_geometry(FrameState* S, const float* lo, const float* hi, int n_ref, int cell_budget) {
+__device__ void set_geometry(FrameState* S, const float* lo, const float* hi, int n_ref, int cell_budget,
+                             int per_cell = kRefsPerCell) {
   float ext[3];
   double vol = 1.0;
   for (int d = 0; d < 3; d++) {
@@ -238,7 +179,7 @@ __device__ void set_geometry(FrameState* S, const float* lo, const float* hi, in
   // about kRefsPerCell references per cell: the neighbours a supervoxel keeps then usually
   // lie within the first ring of cells around the query
   const int budget = max(cell_budget - 1, 1);
-  const int target = max(1, min(budget, n_ref / kRefsPerCell));
+  const int target = max(1, min(budget, n_ref / per_cell));
   float h = (float)cbrt(vol / target);
   int dims[3] = {1, 1, 1};
   for (int guard = 0; guard < 400; guard++) {
@@ -2593,186 +2534,599 @@ void launch_export(const DevPlan& P, cudaStream_t st) { k_export<<<P.max_gchunks
 
 
 // ---------------------------------------------------------------------------
-// Standalone exact kNN (tgmm_knn): the same grid search over one point set.
+// Standalone exact kNN (tgmm_knn, tgmm_knn_k, tgmm_knn_noalloc): a uniform grid over one
+// point set, then the queries.
+//   k_sa_bounds  the queries' bounding box and the grid over it (many blocks, the last one
+//                to finish sets the geometry);
+//   k_sa_count   each reference point's cell and its place within the cell;
+//   k_sa_start   each cell's place in the sorted references (cells in any order: the search
+//                orders by (distance, index), so no scan over the cells is needed);
+//   k_sa_fill    the references into their places;
+//   k_sa_query   G lanes per query.
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(1024) k_sa_geometry(const float* q, int64_t nq, float s0, float s1, float s2,
-                                                      int nref, int budget, FrameState* S) {
-  __shared__ float smin[3][32], smax[3][32];
+
+// Scratch of one search over nref points, carved from one buffer (the first kSaClear +
+// 4 * budget bytes start at zero).
+struct SaScratch {
+  FrameState* S;   // the grid geometry (lo, h, inv_h, dims, n_cells)
+  unsigned* box;   // keys of the box (see box_key), arrived blocks, next free place
+  int* cnt;        // [budget] references per cell
+  int* start;      // [budget] the cell's first place
+  int2* place;     // [nref] cell (-1: in none) and place within it
+  float4* refs;    // [nref] coordinates and index, cell by cell
+};
+static_assert(sizeof(FrameState) <= kSaBox, "the grid geometry record fits its part of the scratch header");
+
+static SaScratch sa_carve(char* buf, int32_t nref) {
+  SaScratch w;
+  w.S = (FrameState*)buf;
+  w.box = (unsigned*)(buf + kSaBox);
+  w.cnt = (int*)(buf + kSaClear);
+  w.start = (int*)(buf + knn_scratch_start(nref));
+  w.place = (int2*)(buf + knn_scratch_place(nref));
+  w.refs = (float4*)(buf + knn_scratch_refs(nref));
+  return w;
+}
+
+// Floats as unsigned keys in the same order; the key of the smallest is above 0, so that a
+// cleared word is the identity of a maximum (minima are kept as the maxima of ~key).
+__device__ __forceinline__ unsigned box_key(float f) {
+  const unsigned b = __float_as_uint(f);
+  return b & 0x80000000u ? ~b : b | 0x80000000u;
+}
+__device__ __forceinline__ float box_value(unsigned k) {
+  return __uint_as_float(k & 0x80000000u ? k & 0x7fffffffu : ~k);
+}
+
+// Bounded by the read of the queries (12 bytes each); one block took 187 us for 1.43 M
+// queries, the whole device 5-6 us.  Non-finite coordinates are left out of the box.
+__global__ void __launch_bounds__(256) k_sa_bounds(const float* __restrict__ q, int64_t nq, float s0, float s1,
+                                                   float s2, int nref, int budget, int per_cell, SaScratch w) {
+  __shared__ unsigned sm[6][8];
   const float sc[3] = {s0, s1, s2};
-  float lo[3] = {kInfF, kInfF, kInfF}, hi[3] = {-kInfF, -kInfF, -kInfF};
-  for (int64_t i = threadIdx.x; i < nq; i += blockDim.x)
+  unsigned lo[3] = {0, 0, 0}, hi[3] = {0, 0, 0};  // lo: the largest ~key
+#pragma unroll 4
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < nq; i += (int64_t)gridDim.x * blockDim.x)
+#pragma unroll
     for (int d = 0; d < 3; d++) {
       const float y = q[d * nq + i] * sc[d];
       if (!isfinite(y)) continue;
-      lo[d] = fminf(lo[d], y);
-      hi[d] = fmaxf(hi[d], y);
+      const unsigned k = box_key(y);
+      lo[d] = max(lo[d], ~k);
+      hi[d] = max(hi[d], k);
     }
-  for (int d = 0; d < 3; d++)
-    for (int o = 16; o > 0; o >>= 1) {
-      lo[d] = fminf(lo[d], __shfl_xor_sync(0xffffffffu, lo[d], o));
-      hi[d] = fmaxf(hi[d], __shfl_xor_sync(0xffffffffu, hi[d], o));
+  const int wp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+#pragma unroll
+  for (int d = 0; d < 3; d++) {
+    lo[d] = __reduce_max_sync(0xffffffffu, lo[d]);
+    hi[d] = __reduce_max_sync(0xffffffffu, hi[d]);
+    if (lane == 0) {
+      sm[d][wp] = lo[d];
+      sm[3 + d][wp] = hi[d];
     }
-  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (lane == 0)
-    for (int d = 0; d < 3; d++) {
-      smin[d][w] = lo[d];
-      smax[d][w] = hi[d];
-    }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    for (int d = 0; d < 3; d++) {
-      lo[d] = smin[d][0];
-      hi[d] = smax[d][0];
-      for (int i = 1; i < (int)(blockDim.x >> 5); i++) {
-        lo[d] = fminf(lo[d], smin[d][i]);
-        hi[d] = fmaxf(hi[d], smax[d][i]);
-      }
-      if (!(lo[d] <= hi[d])) lo[d] = hi[d] = 0.0f;
-    }
-    set_geometry(S, lo, hi, nref, budget);
   }
+  __syncthreads();
+  if (threadIdx.x < 6) {
+    unsigned m = 0;
+#pragma unroll
+    for (int i = 0; i < 8; i++) m = max(m, sm[threadIdx.x][i]);
+    if (m) atomicMax(&w.box[threadIdx.x], m);
+    __threadfence();
+  }
+  __syncthreads();
+  if (threadIdx.x != 0) return;
+  if (atomicAdd(&w.box[6], 1u) != gridDim.x - 1) return;
+  __threadfence();
+  float flo[3], fhi[3];
+  for (int d = 0; d < 3; d++) {
+    const unsigned a = __ldcg(&w.box[d]), b = __ldcg(&w.box[3 + d]);
+    flo[d] = fhi[d] = 0.0f;  // no finite coordinate
+    if (b != 0) {
+      flo[d] = box_value(~a);
+      fhi[d] = box_value(b);
+    }
+  }
+  set_geometry(w.S, flo, fhi, nref, budget, per_cell);
 }
 
 // Reference point k, coordinate d, sits at ref[k * step + d * comp]: AoS xyz (step 3,
 // comp 1) or SoA x-block, y-block, z-block (step 1, comp nref).
-__global__ void k_sa_count(const float* ref, int nref, int step, int64_t comp, float s0, float s1, float s2,
-                           const FrameState* S, int* cnt, int* rcell) {
+__global__ void __launch_bounds__(256) k_sa_count(const float* __restrict__ ref, int nref, int step, int64_t comp,
+                                                  float s0, float s1, float s2, SaScratch w) {
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= nref) return;
   const float* rk = ref + (int64_t)k * step;
   const float ys[3] = {rk[0] * s0, rk[comp] * s1, rk[2 * comp] * s2};
-  int cell = 0;
+  int2 p = make_int2(0, 0);
   for (int d = 0; d < 3; d++)
-    if (!isfinite(ys[d]) || fabsf(ys[d]) >= 1e25f) cell = -1;
-  if (cell == 0) {
-    const int cx = cell_coord(ys[0], S->lo[0], S->inv_h, S->dims[0]);
-    const int cy = cell_coord(ys[1], S->lo[1], S->inv_h, S->dims[1]);
-    const int cz = cell_coord(ys[2], S->lo[2], S->inv_h, S->dims[2]);
-    cell = (cz * S->dims[1] + cy) * S->dims[0] + cx;
-    atomicAdd(&cnt[cell], 1);
+    if (!isfinite(ys[d]) || fabsf(ys[d]) >= 1e25f) p.x = -1;
+  if (p.x == 0) {
+    const int cx = cell_coord(ys[0], w.S->lo[0], w.S->inv_h, w.S->dims[0]);
+    const int cy = cell_coord(ys[1], w.S->lo[1], w.S->inv_h, w.S->dims[1]);
+    const int cz = cell_coord(ys[2], w.S->lo[2], w.S->inv_h, w.S->dims[2]);
+    p.x = (cz * w.S->dims[1] + cy) * w.S->dims[0] + cx;
+    p.y = atomicAdd(&w.cnt[p.x], 1);
   }
-  rcell[k] = cell;
+  w.place[k] = p;
 }
 
-__global__ void __launch_bounds__(1024) k_sa_scan(const FrameState* S, int* cnt, int* start, int* cur) {
-  __shared__ int scan[1024];
-  const int n = S->n_cells;
-  const int per = (n + blockDim.x - 1) / blockDim.x;
-  const int b0 = min(n, (int)threadIdx.x * per), b1 = min(n, b0 + per);
-  int local = 0;
-  for (int i = b0; i < b1; i++) local += cnt[i];
-  scan[threadIdx.x] = local;
-  __syncthreads();
-  for (int off = 1; off < (int)blockDim.x; off <<= 1) {
-    int v = (threadIdx.x >= (unsigned)off) ? scan[threadIdx.x - off] : 0;
-    __syncthreads();
-    scan[threadIdx.x] += v;
-    __syncthreads();
-  }
-  int run = scan[threadIdx.x] - local;
-  for (int i = b0; i < b1; i++) {
-    start[i] = run;
-    cur[i] = run;
-    run += cnt[i];
-  }
-  if (threadIdx.x == blockDim.x - 1) start[n] = scan[blockDim.x - 1];
-}
-
-__global__ void k_sa_fill(const float* ref, int nref, int step, int64_t comp, const int* rcell, int* cur,
-                          float4* refs) {
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= nref || rcell[k] < 0) return;
-  const int pos = atomicAdd(&cur[rcell[k]], 1);
-  const float* rk = ref + (int64_t)k * step;
-  refs[pos] = make_float4(rk[0], rk[comp], rk[2 * comp], __int_as_float(k));
-}
-
-__global__ void k_sa_query(const float* q, int64_t nq, const float* ref, int nref, float s0, float s1, float s2,
-                           const FrameState* S, const int* start, const float4* refs, int32_t* ind) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= nq) return;
-  const float sc[3] = {s0, s1, s2};
-  const float q0 = q[i], q1 = q[nq + i], q2 = q[2 * nq + i];
-  GridGeom g;
-  for (int d = 0; d < 3; d++) {
-    g.lo[d] = S->lo[d];
-    g.dims[d] = S->dims[d];
-  }
-  g.h = S->h;
-  g.inv_h = S->inv_h;
-  Top5 t;
-  top5_init(t);
-  knn_grid_search<kJ>(q0, q1, q2, sc, g, start, refs, t);
-  if (!(t.d[kJ - 1] < kInfF)) {
-    top5_init(t);
-    for (int k = 0; k < nref; k++) top5_insert(t, knn_dist(q0, q1, q2, ref[3 * k], ref[3 * k + 1], ref[3 * k + 2], sc), k);
-  }
-  for (int j = 0; j < kJ; j++) ind[(int64_t)j * nq + i] = t.i[j];
-}
-
-// The K nearest (K <= kMaxK) of each query with their squared scaled distances, for the
-// tracking graph's supervoxel kNN: the same grid search, the same exact fallback scan when
-// fewer than K finite distances were found, (distance, index) order; a slot with no
-// reference point closer than 1e32 (squared) gets index -1 and distance 1e32.
-template <int K>
-__global__ void k_sa_query_k(const float* q, int64_t nq, const float* ref, int nref, int step, int64_t comp,
-                             float s0, float s1, float s2, const FrameState* S, const int* start, const float4* refs,
-                             int32_t* ind, float* dist) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= nq) return;
-  const float sc[3] = {s0, s1, s2};
-  const float q0 = q[i], q1 = q[nq + i], q2 = q[2 * nq + i];
-  GridGeom g;
-  for (int d = 0; d < 3; d++) {
-    g.lo[d] = S->lo[d];
-    g.dims[d] = S->dims[d];
-  }
-  g.h = S->h;
-  g.inv_h = S->inv_h;
-  TopN<K> t;
-  topn_init<K>(t);
-  knn_grid_search<K>(q0, q1, q2, sc, g, start, refs, t);
-  if (!(t.d[K - 1] < kInfF)) {
-    topn_init<K>(t);
-    for (int k = 0; k < nref; k++) {
-      const float* rk = ref + (int64_t)k * step;
-      topn_insert<K>(t, knn_dist(q0, q1, q2, rk[0], rk[comp], rk[2 * comp], sc), k);
+// A warp per x-row of cells: the row's references get one contiguous range, its cells in
+// order, the rows in any order (the searches order by (distance, index)).
+__global__ void __launch_bounds__(256) k_sa_start(SaScratch w) {
+  const int lane = threadIdx.x & 31;
+  const int nx = w.S->dims[0], rows = w.S->dims[1] * w.S->dims[2];
+  for (int r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < rows; r += (gridDim.x * blockDim.x) >> 5) {
+    int total = 0;
+    for (int x = lane; x < nx; x += 32) total += w.cnt[r * nx + x];
+    total = __reduce_add_sync(0xffffffffu, total);
+    int base = 0;
+    if (lane == 0 && total > 0) base = (int)atomicAdd(&w.box[7], (unsigned)total);
+    base = __shfl_sync(0xffffffffu, base, 0);
+    for (int x0 = 0; x0 < nx; x0 += 32) {
+      const int x = x0 + lane;
+      const int m = x < nx ? w.cnt[r * nx + x] : 0;
+      int inc = m;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= o) inc += v;
+      }
+      if (x < nx) w.start[r * nx + x] = base + inc - m;
+      base += __shfl_sync(0xffffffffu, inc, 31);
     }
   }
+}
+
+__global__ void __launch_bounds__(256) k_sa_fill(const float* __restrict__ ref, int nref, int step, int64_t comp,
+                                                 SaScratch w) {
+  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= nref) return;
+  const int2 p = w.place[k];
+  if (p.x < 0) return;
+  const float* rk = ref + (int64_t)k * step;
+  w.refs[w.start[p.x] + p.y] = make_float4(rk[0], rk[comp], rk[2 * comp], __int_as_float(k));
+}
+
+// Where a query sits in the grid: its cell, the gaps to that cell's faces, and the float
+// rounding of the scaled coordinates and faces (eps0; distances of d add 1e-6 d).
+struct SaPlace {
+  int c[3];
+  float f0[3], f1[3];  // gaps to the cell's lower and upper faces
+  float delta, eps0;   // the smallest gap; the rounding
+  __device__ __forceinline__ SaPlace(float q0, float q1, float q2, const float* s, const GridGeom& g) {
+    const float y[3] = {q0 * s[0], q1 * s[1], q2 * s[2]};
+    float ymax = 0.0f;
+    delta = kInfF;
+#pragma unroll
+    for (int a = 0; a < 3; a++) {
+      c[a] = cell_coord(y[a], g.lo[a], g.inv_h, g.dims[a]);
+      f0[a] = y[a] - (g.lo[a] + c[a] * g.h);
+      f1[a] = (g.lo[a] + (c[a] + 1) * g.h) - y[a];
+      delta = fminf(delta, fminf(f0[a], f1[a]));
+      ymax = fmaxf(ymax, fabsf(y[a]));
+    }
+    delta = fmaxf(delta, 0.0f);
+    eps0 = 4e-3f + 1e-6f * ymax;
+  }
+  // A squared distance below which every reference lies in the cells at Chebyshev distance
+  // <= r (0: none is known).  References outside the box sit in the boundary cells, farther
+  // from a query inside it than those cells.
+  __device__ __forceinline__ float bound2(int r, float h) const {
+    const float lb = r * h + delta, m = lb - (eps0 + 1e-6f * lb);
+    return m > 0.0f ? m * m : 0.0f;
+  }
+  // squared lower bound of the distance along axis a to the cells at offset o
+  __device__ __forceinline__ float gap2(int a, int o, float h) const {
+    const float gap = o < 0 ? f0[a] + (float)(-o - 1) * h : f1[a] + (float)(o - 1) * h;
+    const float m = fmaxf(gap - eps0 - 1e-6f * gap, 0.0f);
+    return o == 0 ? 0.0f : m * m;
+  }
+};
+
+template <typename F>
+__device__ __forceinline__ void sa_scan_cell(const SaScratch& w, int cell, float q0, float q1, float q2, const float* s,
+                                             F take) {
+  const int b = w.start[cell], e = b + w.cnt[cell];
+  for (int k = b; k < e; ++k) {
+    const float4 rr = w.refs[k];
+    take(knn_dist(q0, q1, q2, rr.x, rr.y, rr.z, s), __float_as_int(rr.w));
+  }
+}
+
+// The N nearest of one query by one thread: rings of cells at growing Chebyshev distance
+// around the query's cell, passing over cells farther than the N-th distance so far.  Ends
+// when the N-th distance is strictly below the bound of every cell not visited.
+template <int N>
+__device__ __noinline__ void sa_search_thread(float q0, float q1, float q2, const float* s, const GridGeom& g,
+                                              const SaScratch& w, TopN<N>& best) {
+  const SaPlace p(q0, q1, q2, s, g);
+  topn_init<N>(best);
+  const int maxr = max(g.dims[0], max(g.dims[1], g.dims[2]));
+  for (int r = 0; r <= maxr; ++r) {
+    const int z0 = max(p.c[2] - r, 0), z1 = min(p.c[2] + r, g.dims[2] - 1);
+    const int y0 = max(p.c[1] - r, 0), y1 = min(p.c[1] + r, g.dims[1] - 1);
+    for (int z = z0; z <= z1; ++z) {
+      const float gz = p.gap2(2, z - p.c[2], g.h);
+      if (gz > best.d[N - 1]) continue;
+      const bool zedge = (z == p.c[2] - r) || (z == p.c[2] + r);
+      for (int yy = y0; yy <= y1; ++yy) {
+        const float gy = gz + p.gap2(1, yy - p.c[1], g.h);
+        if (gy > best.d[N - 1]) continue;
+        const bool edge = zedge || (yy == p.c[1] - r) || (yy == p.c[1] + r);
+        const int row = (z * g.dims[1] + yy) * g.dims[0];
+        const int step = edge || r == 0 ? 1 : 2 * r;
+        for (int x = p.c[0] - r; x <= p.c[0] + r; x += step) {
+          if (x < 0 || x >= g.dims[0] || gy + p.gap2(0, x - p.c[0], g.h) > best.d[N - 1]) continue;
+          sa_scan_cell(w, row + x, q0, q1, q2, s, [&](float d, int id) { topn_insert<N>(best, d, id); });
+        }
+      }
+    }
+    if (best.d[N - 1] < p.bound2(r, g.h)) break;
+  }
+}
+
+// The same by the G lanes of a group, a ring at a time from the 27 cells around the query:
+// the lanes split a ring's cells and merge their lists after it.
+template <int G, int N>
+__device__ __noinline__ void sa_search_group(float q0, float q1, float q2, const float* s, const GridGeom& g,
+                                             const SaScratch& w, TopN<N>& best, int gl, unsigned gmask) {
+  const SaPlace p(q0, q1, q2, s, g);
+  topn_init<N>(best);
+  const int maxr = max(1, max(g.dims[0], max(g.dims[1], g.dims[2])));
+  for (int r = 1; r <= maxr; ++r) {
+    TopN<N> t;
+    topn_init<N>(t);
+    const float td = best.d[N - 1];
+    const int ti = best.i[N - 1];
+    const int side = 2 * r + 1, cube = side * side * side;
+    for (int idx = gl; idx < cube; idx += G) {
+      const int dx = idx % side - r, dy = (idx / side) % side - r, dz = idx / (side * side) - r;
+      if (r > 1 && max(abs(dx), max(abs(dy), abs(dz))) != r) continue;
+      if (p.gap2(0, dx, g.h) + p.gap2(1, dy, g.h) + p.gap2(2, dz, g.h) > td) continue;
+      const int x = p.c[0] + dx, yy = p.c[1] + dy, z = p.c[2] + dz;
+      if (x < 0 || yy < 0 || z < 0 || x >= g.dims[0] || yy >= g.dims[1] || z >= g.dims[2]) continue;
+      sa_scan_cell(w, (z * g.dims[1] + yy) * g.dims[0] + x, q0, q1, q2, s, [&](float d, int id) {
+        if (!before(td, ti, d, id)) topn_insert<N>(t, d, id);
+      });
+    }
+    if (gl == 0) {
+#pragma unroll
+      for (int j = 0; j < N; j++) topn_insert<N>(t, best.d[j], best.i[j]);
+    }
+    TopN<N> merged;
+    group_merge_topn<G, N>(t, merged, gmask);
+    best = merged;
+    if (best.d[N - 1] < p.bound2(r, g.h)) break;
+  }
+}
+
+__device__ __forceinline__ GridGeom sa_geometry(const SaScratch& w) {
+  GridGeom g;
+  for (int d = 0; d < 3; d++) {
+    g.lo[d] = w.S->lo[d];
+    g.dims[d] = w.S->dims[d];
+  }
+  g.h = w.S->h;
+  g.inv_h = w.S->inv_h;
+  return g;
+}
+
+// Slot j of query i.  kMark (tgmm_knn_k): a slot with no reference closer than 1e32 (squared)
+// gets index -1 and distance 1e32; else every slot holds its index.
+template <bool kMark>
+__device__ __forceinline__ void sa_write(int32_t* ind, float* dist, int64_t nq, int64_t i, int j, float d, int id) {
+  const bool real = !kMark || (id != 0x7fffffff && d < 1e32f);
+  ind[(int64_t)j * nq + i] = real ? id : -1;
+  if (kMark && dist) dist[(int64_t)j * nq + i] = real ? d : 1e32f;
+}
+
+// References per grid cell for searches of K: the sphere of the cell's side then holds about
+// 2 K references on average.
+constexpr int sa_per_cell(int K) { return K <= 4 ? 2 : (K + 1) / 2; }
+// The first radius of a search, expected to hold 2 K references at the grid's mean density.
+template <int K>
+__device__ __forceinline__ float sa_first_radius(float h) {
+  return h * cbrtf(2.0f * K * (3.0f / (4.0f * 3.14159265f)) / sa_per_cell(K));
+}
+// The next radius after n references were found where K to kSaKeep are wanted.
+template <int K>
+__device__ __forceinline__ float sa_next_radius(float rad, int n) {
+  const float f = cbrtf((n < K ? 2.0f * K : 1.5f * K) / ((float)n + 0.5f));
+  return rad * (n < K ? fminf(fmaxf(f, 1.25f), 2.0f) : fminf(f, 0.9f));
+}
+
+constexpr int kSaKeep = 64;       // references kept per query of a group
+constexpr int kSaKeepWarp = 128;  // references kept per warp of queries
+constexpr int kSaTries = 4;       // radii tried before the ring search
+constexpr int kSaRounds = 4;      // sets of near queries a warp is split into before it
+constexpr int kSaSet = 4;         // fewest queries of a set
+constexpr int kSaRows = 256;      // rows of cells scanned at most in one try
+
+// The references within `rad` of the box [lo, hi] (scaled space), collected by the G lanes of a
+// group into keep[0 .. cap) in any order: for a point box (kPoint) as (distance, index) of those
+// closer than rad by the exact distance, else the references themselves.  Rows of cells are
+// contiguous in w.refs; a row is passed over when its gap to the box along y and z is rad or
+// more.  Returns how many there are (more than cap: the rest were dropped), or -1 when the rows
+// are too many.  References outside the grid's box sit in its boundary cells, farther from a
+// box inside it than those cells.  Every lane of the group takes part in every step.
+template <int G, bool kPoint, typename T>
+__device__ __forceinline__ int sa_collect(const float* qv, const float* lo, const float* hi, float rad, float eps0,
+                                          const float* s, const GridGeom& g, const SaScratch& w, T* keep, int cap,
+                                          int gl, unsigned gmask) {
+  int c0[3], c1[3];
+#pragma unroll
+  for (int a = 0; a < 3; a++) {
+    const float m = rad + 2.0f * eps0;
+    c0[a] = cell_coord(lo[a] - m, g.lo[a], g.inv_h, g.dims[a]);
+    c1[a] = cell_coord(hi[a] + m, g.lo[a], g.inv_h, g.dims[a]);
+  }
+  if ((int64_t)(c1[1] - c0[1] + 1) * (c1[2] - c0[2] + 1) > kSaRows) return -1;
+  const float r2 = rad * rad;
+  // squared lower bound of a gap of `v` along one axis
+  auto sq = [&](float v) {
+    const float m = fmaxf(v - eps0 - 1e-6f * v, 0.0f);
+    return m * m;
+  };
+  int n = 0;
+  const unsigned below = (1u << (threadIdx.x & 31)) - 1u;
+  for (int z = c0[2]; z <= c1[2]; z++) {
+    const float fz = g.lo[2] + z * g.h;
+    const float gz = sq(fmaxf(lo[2] - (fz + g.h), fz - hi[2]));
+    if (!(gz < r2)) continue;
+    for (int y = c0[1]; y <= c1[1]; y++) {
+      const float fy = g.lo[1] + y * g.h;
+      if (!(gz + sq(fmaxf(lo[1] - (fy + g.h), fy - hi[1])) < r2)) continue;
+      const int row = (z * g.dims[1] + y) * g.dims[0];
+      const int b = w.start[row + c0[0]], e = w.start[row + c1[0]] + w.cnt[row + c1[0]];
+      for (int k0 = b; k0 < e; k0 += G) {
+        const int k = k0 + gl;
+        bool take = false;
+        float4 rr = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        float d = 0.0f;
+        if (k < e) {
+          rr = w.refs[k];
+          if (kPoint) {
+            d = knn_dist(qv[0], qv[1], qv[2], rr.x, rr.y, rr.z, s);
+          } else {
+            const float yr[3] = {rr.x * s[0], rr.y * s[1], rr.z * s[2]};
+#pragma unroll
+            for (int a = 0; a < 3; a++) d += sq(fmaxf(lo[a] - yr[a], yr[a] - hi[a]));
+          }
+          take = d < r2;
+        }
+        const unsigned m = __ballot_sync(gmask, take) & gmask;
+        const int at = n + __popc(m & below);
+        if (take && at < cap) {
+          if constexpr (kPoint)
+            keep[at] = make_float2(d, rr.w);
+          else
+            keep[at] = rr;
+        }
+        n += __popc(m);
+      }
+    }
+  }
+  return n;
+}
+
+// The K nearest of the n references kept for a warp, in (distance, index) order.  First the
+// K + 1 smallest keys -- the distance's upper bits with the place in `keep` below them, two
+// instructions a level -- then the K of them in exact order.  Returns false when the K-th and
+// the next key share their distance bits, which leaves open which of them belongs.
+template <int K>
+__device__ __forceinline__ bool sa_select(const float* qv, const float* s, const float4* keep, int n, TopN<K>& t) {
+  static_assert(kSaKeepWarp == 128, "seven bits of place in a key");
+  unsigned key[K + 1];
+#pragma unroll
+  for (int j = 0; j <= K; j++) key[j] = 0xffffffffu;
+#pragma unroll 4
+  for (int k = 0; k < n; k++) {
+    const float4 rr = keep[k];
+    const float d = knn_dist(qv[0], qv[1], qv[2], rr.x, rr.y, rr.z, s);
+    unsigned v = (__float_as_uint(d) & ~127u) | (unsigned)k;
+#pragma unroll
+    for (int j = 0; j <= K; j++) {
+      const unsigned lo = min(key[j], v);
+      v = max(key[j], v);
+      key[j] = lo;
+    }
+  }
+  topn_init<K>(t);
 #pragma unroll
   for (int j = 0; j < K; j++) {
-    const bool real = t.i[j] != 0x7fffffff && t.d[j] < 1e32f;
-    ind[(int64_t)j * nq + i] = real ? t.i[j] : -1;
-    if (dist) dist[(int64_t)j * nq + i] = real ? t.d[j] : 1e32f;
+    const float4 rr = keep[key[j] & 127u];
+    topn_insert<K>(t, knn_dist(qv[0], qv[1], qv[2], rr.x, rr.y, rr.z, s), __float_as_int(rr.w));
   }
+  return (key[K - 1] & ~127u) != (key[K] & ~127u);
+}
+
+// A warp's 32 consecutive queries together, for queries whose neighbours in the array are near
+// one another (the voxels of a supervoxel): the queries within a cell's side of the first
+// collect the references within a radius of their bounding box, then each lane orders them for
+// its own query.  A lane's K nearest are exact when its K-th is closer than the radius, since
+// every reference not collected is at least the radius away from the box; the largest K-th
+// distance is the next radius, which serves all of them.  Queries elsewhere (the warp runs into
+// the next supervoxel) are the next set; what is left over (scattered queries, crowded cells,
+// distances too close to tell apart by their keys) runs the ring search.  1.43 M voxels against
+// 2000 references: 133 us, 71% of the issue slots busy (a thread per query: 239 us).
+template <int K, bool kMark>
+__global__ void __launch_bounds__(128) k_sa_query_warp(const float* __restrict__ q, int64_t nq,
+                                                       const float* __restrict__ ref, int nref, int step,
+                                                       int64_t comp, float s0, float s1, float s2, SaScratch w,
+                                                       int32_t* ind, float* dist) {
+  __shared__ float4 s_keep[4][kSaKeepWarp];
+  const int lane = threadIdx.x & 31;
+  float4* keep = s_keep[threadIdx.x >> 5];
+  const int64_t i0 = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) & ~(int64_t)31;
+  if (i0 >= nq) return;  // whole warps leave
+  const int64_t i = min(i0 + lane, nq - 1);  // the last warp's spare lanes repeat its last query
+  const float sc[3] = {s0, s1, s2};
+  const float qv[3] = {q[i], q[nq + i], q[2 * nq + i]};
+  const float yq[3] = {qv[0] * s0, qv[1] * s1, qv[2] * s2};
+  const GridGeom g = sa_geometry(w);
+  TopN<K> t;
+  topn_init<K>(t);
+  const bool fin = isfinite(yq[0]) && isfinite(yq[1]) && isfinite(yq[2]);
+  bool waits = fin, done = false;
+  for (int round = 0; round < kSaRounds; round++) {
+    const unsigned left = __ballot_sync(0xffffffffu, waits);
+    if (!left) break;
+    const int lead = __ffs(left) - 1;
+    bool mine = waits;
+#pragma unroll
+    for (int a = 0; a < 3; a++) {
+      const float yl = __shfl_sync(0xffffffffu, yq[a], lead);  // every lane takes part
+      mine = mine && fabsf(yq[a] - yl) <= g.h;
+    }
+    if (__popc(__ballot_sync(0xffffffffu, mine)) < kSaSet) break;  // scattered queries
+    float lo[3], hi[3], ymax = 0.0f;
+#pragma unroll
+    for (int a = 0; a < 3; a++) {
+      const unsigned k = box_key(yq[a]);
+      lo[a] = box_value(~__reduce_max_sync(0xffffffffu, mine ? ~k : 0u));
+      hi[a] = box_value(__reduce_max_sync(0xffffffffu, mine ? k : 0u));
+      ymax = fmaxf(ymax, fmaxf(fabsf(lo[a]), fabsf(hi[a])));
+    }
+    const float eps0 = 4e-3f + 1e-6f * ymax;
+    float rad = sa_first_radius<K>(g.h);
+    for (int u = 0; u < kSaTries; u++) {
+      const int n = sa_collect<32, false>(qv, lo, hi, rad, eps0, sc, g, w, keep, kSaKeepWarp, lane, 0xffffffffu);
+      __syncwarp();
+      if (n < 0) break;
+      if (n >= K && n <= kSaKeepWarp) {
+        bool tell = true, ok = true;
+        if (mine) {
+          tell = sa_select<K>(qv, sc, keep, n, t);
+          ok = t.d[K - 1] < rad * rad * (1.0f - 2e-6f);
+          done = tell && ok;
+        }
+        if (__all_sync(0xffffffffu, ok)) break;
+        const float far = __uint_as_float(__reduce_max_sync(0xffffffffu, mine ? __float_as_uint(t.d[K - 1]) : 0u));
+        rad = fmaxf(sqrtf(far) * (1.0f + 4e-6f), rad * 1.01f);
+      } else {
+        rad = sa_next_radius<K>(rad, n);
+      }
+      __syncwarp();  // every lane is done with the kept references
+    }
+    __syncwarp();
+    waits = waits && !mine;
+  }
+  if (!done) {
+    sa_search_thread<K>(qv[0], qv[1], qv[2], sc, g, w, t);
+    if (!(t.d[K - 1] < kInfF)) {  // fewer than K finite distances: every reference point
+      topn_init<K>(t);
+      for (int k = 0; k < nref; k++) {
+        const float* rk = ref + (int64_t)k * step;
+        topn_insert<K>(t, knn_dist(qv[0], qv[1], qv[2], rk[0], rk[comp], rk[2 * comp], sc), k);
+      }
+    }
+  }
+  if (i0 + lane < nq)
+#pragma unroll
+    for (int j = 0; j < K; j++) sa_write<kMark>(ind, dist, nq, i, j, t.d[j], t.i[j]);
+}
+
+// A group of G lanes per query, for queries that are scattered or too few to fill the device
+// with a warp per 32: the group collects the references within a radius of the query, and with
+// K to kSaKeep of them each lane ranks its share against all and writes those of rank < K, so
+// that no sorted list is kept.  Radii are tried in turn, then the ring search.  20,019 queries,
+// 20,007 references, K = 10: 48 us, bound by the chain of dependent loads (a thread per query,
+// 625 warps on the device: 195 us).
+template <int G, int K, bool kMark>
+__global__ void __launch_bounds__(128) k_sa_query_group(const float* __restrict__ q, int64_t nq,
+                                                        const float* __restrict__ ref, int nref, int step,
+                                                        int64_t comp, float s0, float s1, float s2, SaScratch w,
+                                                        int32_t* ind, float* dist) {
+  __shared__ float2 s_keep[128 / G][kSaKeep];
+  const int lane = threadIdx.x & 31, gl = lane & (G - 1);
+  float2* keep = s_keep[threadIdx.x / G];
+  const unsigned gmask = G == 32 ? 0xffffffffu : ((1u << G) - 1u) << (lane - gl);
+  const int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / G;
+  if (i >= nq) return;  // whole groups leave together
+  const float sc[3] = {s0, s1, s2};
+  const float qv[3] = {q[i], q[nq + i], q[2 * nq + i]};
+  const float yq[3] = {qv[0] * s0, qv[1] * s1, qv[2] * s2};
+  const GridGeom g = sa_geometry(w);
+  if (isfinite(yq[0]) && isfinite(yq[1]) && isfinite(yq[2])) {
+    const float eps0 = 4e-3f + 1e-6f * fmaxf(fmaxf(fabsf(yq[0]), fabsf(yq[1])), fabsf(yq[2]));
+    float rad = sa_first_radius<K>(g.h);
+    for (int u = 0; u < kSaTries; u++) {
+      const int n = sa_collect<G, true>(qv, yq, yq, rad, eps0, sc, g, w, keep, kSaKeep, gl, gmask);
+      __syncwarp(gmask);
+      if (n < 0) break;
+      if (n >= K && n <= kSaKeep) {
+        for (int a = gl; a < n; a += G) {
+          const float2 e = keep[a];
+          int rank = 0;
+#pragma unroll 4
+          for (int o = 0; o < n; o++) {
+            const float2 f = keep[o];
+            rank += before(f.x, __float_as_int(f.y), e.x, __float_as_int(e.y)) ? 1 : 0;
+          }
+          if (rank < K) sa_write<kMark>(ind, dist, nq, i, rank, e.x, __float_as_int(e.y));
+        }
+        return;
+      }
+      rad = sa_next_radius<K>(rad, n);
+    }
+  }
+  TopN<K> t;
+  sa_search_group<G, K>(qv[0], qv[1], qv[2], sc, g, w, t, gl, gmask);
+  if (!(t.d[K - 1] < kInfF)) {
+    TopN<K> mine;
+    topn_init<K>(mine);
+    for (int k = gl; k < nref; k += G) {
+      const float* rk = ref + (int64_t)k * step;
+      topn_insert<K>(mine, knn_dist(qv[0], qv[1], qv[2], rk[0], rk[comp], rk[2 * comp], sc), k);
+    }
+    group_merge_topn<G, K>(mine, t, gmask);
+  }
+#pragma unroll
+  for (int j = 0; j < K; j++)
+    if (j % G == gl) sa_write<kMark>(ind, dist, nq, i, j, t.d[j], t.i[j]);
+}
+
+// Below this many queries a group of 16 lanes per query, from it on a warp per 32.  Query kernel
+// alone, group / warp: 20,019 queries, K = 10: 48 / 147 us; 60,000: 141 / 196; 200,000 voxels,
+// K = 5: 150 / 82; 1.43 M: 838 / 133.  Groups of 8 and 32: 52 and 47, 150 and 140, 121 and 239.
+constexpr int64_t kSaGroupBelow = 100000;
+
+template <int K, bool kMark>
+static void sa_query(const float* q, int64_t nq, const float* ref, int32_t nref, int step, int64_t comp,
+                     const float scale[3], const SaScratch& w, int32_t* ind, float* dist, cudaStream_t st) {
+  if (nq < kSaGroupBelow)
+    k_sa_query_group<16, K, kMark><<<(unsigned)((nq * 16 + 127) / 128), 128, 0, st>>>(
+        q, nq, ref, nref, step, comp, scale[0], scale[1], scale[2], w, ind, dist);
+  else
+    k_sa_query_warp<K, kMark><<<(unsigned)((nq + 127) / 128), 128, 0, st>>>(
+        q, nq, ref, nref, step, comp, scale[0], scale[1], scale[2], w, ind, dist);
+}
+
+// The grid over the references and the queries' box, in `buf` (knn_grid_scratch_bytes(nref)).
+static cudaError_t sa_build(const float* q, int64_t nq, const float* ref, int32_t nref, int step, int64_t comp,
+                            const float scale[3], int K, char* buf, SaScratch* w, cudaStream_t st) {
+  *w = sa_carve(buf, nref);
+  const int budget = 2 * nref + 2;
+  cudaError_t e = cudaMemsetAsync(buf + kSaBox, 0, kSaClear - kSaBox + 4 * (size_t)budget, st);
+  if (e != cudaSuccess) return e;
+  const int64_t nb = (nq + 1023) / 1024;
+  k_sa_bounds<<<(unsigned)(nb < 592 ? nb : 592), 256, 0, st>>>(q, nq, scale[0], scale[1], scale[2], nref, budget,
+                                                             sa_per_cell(K), *w);
+  const int gb = (nref + 255) / 256;
+  k_sa_count<<<gb, 256, 0, st>>>(ref, nref, step, comp, scale[0], scale[1], scale[2], *w);
+  k_sa_start<<<(unsigned)std::min(592, (budget + 255) / 256), 256, 0, st>>>(*w);
+  k_sa_fill<<<gb, 256, 0, st>>>(ref, nref, step, comp, *w);
+  return cudaGetLastError();
 }
 
 cudaError_t knn_grid_standalone(const float* q, int64_t nq, const float* ref, int32_t nref, const float scale[3],
                                 int32_t* ind, cudaStream_t st) {
-  const int budget = 2 * nref + 2;
   char* buf = nullptr;
-  const size_t off_state = 0, off_cnt = 256, off_start = off_cnt + 4 * (size_t)budget,
-               off_cur = off_start + 4 * ((size_t)budget + 1), off_rc = off_cur + 4 * (size_t)budget,
-               off_refs = (off_rc + 4 * (size_t)nref + 255) / 256 * 256, total = off_refs + 16 * (size_t)nref;
-  cudaError_t e = cudaMallocAsync((void**)&buf, total, st);
+  cudaError_t e = cudaMallocAsync((void**)&buf, knn_grid_scratch_bytes(nref), st);
   if (e != cudaSuccess) return e;
-  FrameState* S = (FrameState*)(buf + off_state);
-  int* cnt = (int*)(buf + off_cnt);
-  int* start = (int*)(buf + off_start);
-  int* cur = (int*)(buf + off_cur);
-  int* rc = (int*)(buf + off_rc);
-  float4* refs = (float4*)(buf + off_refs);
-  cudaMemsetAsync(cnt, 0, 4 * (size_t)budget, st);
-  k_sa_geometry<<<1, 1024, 0, st>>>(q, nq, scale[0], scale[1], scale[2], nref, budget, S);
-  const int gb = (nref + 255) / 256;
-  k_sa_count<<<gb, 256, 0, st>>>(ref, nref, 3, 1, scale[0], scale[1], scale[2], S, cnt, rc);
-  k_sa_scan<<<1, 1024, 0, st>>>(S, cnt, start, cur);
-  k_sa_fill<<<gb, 256, 0, st>>>(ref, nref, 3, 1, rc, cur, refs);
-  k_sa_query<<<(unsigned)((nq + 127) / 128), 128, 0, st>>>(q, nq, ref, nref, scale[0], scale[1], scale[2], S, start,
-                                                          refs, ind);
-  e = cudaGetLastError();
-  cudaFreeAsync(buf, st);
-  return e;
+  e = knn_grid_in_scratch(q, nq, ref, nref, scale, ind, st, buf);
+  const cudaError_t ef = cudaFreeAsync(buf, st);
+  return e != cudaSuccess ? e : ef;
 }
 
 // The K-nearest grid search (1 <= K <= kMaxK) over reference points in AoS or SoA layout
@@ -2781,75 +3135,37 @@ cudaError_t knn_grid_topk(const float* q, int64_t nq, const float* ref, int32_t 
                           const float scale[3], int32_t* ind, float* dist, cudaStream_t st) {
   const int step = soa ? 1 : 3;
   const int64_t comp = soa ? nref : 1;
-  const int budget = 2 * nref + 2;
   char* buf = nullptr;
-  const size_t off_state = 0, off_cnt = 256, off_start = off_cnt + 4 * (size_t)budget,
-               off_cur = off_start + 4 * ((size_t)budget + 1), off_rc = off_cur + 4 * (size_t)budget,
-               off_refs = (off_rc + 4 * (size_t)nref + 255) / 256 * 256, total = off_refs + 16 * (size_t)nref;
-  cudaError_t e = cudaMallocAsync((void**)&buf, total, st);
+  cudaError_t e = cudaMallocAsync((void**)&buf, knn_grid_scratch_bytes(nref), st);
   if (e != cudaSuccess) return e;
-  FrameState* S = (FrameState*)(buf + off_state);
-  int* cnt = (int*)(buf + off_cnt);
-  int* start = (int*)(buf + off_start);
-  int* cur = (int*)(buf + off_cur);
-  int* rc = (int*)(buf + off_rc);
-  float4* refs = (float4*)(buf + off_refs);
-  cudaMemsetAsync(cnt, 0, 4 * (size_t)budget, st);
-  k_sa_geometry<<<1, 1024, 0, st>>>(q, nq, scale[0], scale[1], scale[2], nref, budget, S);
-  const int gb = (nref + 255) / 256;
-  k_sa_count<<<gb, 256, 0, st>>>(ref, nref, step, comp, scale[0], scale[1], scale[2], S, cnt, rc);
-  k_sa_scan<<<1, 1024, 0, st>>>(S, cnt, start, cur);
-  k_sa_fill<<<gb, 256, 0, st>>>(ref, nref, step, comp, rc, cur, refs);
-  const unsigned grid = (unsigned)((nq + 127) / 128);
-  switch (K) {
-#define TGMM_TOPK_CASE(KK)                                                                                     \
-  case KK:                                                                                                   \
-    k_sa_query_k<KK><<<grid, 128, 0, st>>>(q, nq, ref, nref, step, comp, scale[0], scale[1], scale[2], S, start, \
-                                           refs, ind, dist);                                                 \
+  SaScratch w;
+  e = sa_build(q, nq, ref, nref, step, comp, scale, K, buf, &w, st);
+  if (e == cudaSuccess) {
+    switch (K) {
+#define TGMM_TOPK_CASE(KK)                                                              \
+  case KK:                                                                              \
+    sa_query<KK, true>(q, nq, ref, nref, step, comp, scale, w, ind, dist, st);          \
     break;
-    TGMM_TOPK_CASE(1) TGMM_TOPK_CASE(2) TGMM_TOPK_CASE(3) TGMM_TOPK_CASE(4) TGMM_TOPK_CASE(5) TGMM_TOPK_CASE(6)
-    TGMM_TOPK_CASE(7) TGMM_TOPK_CASE(8) TGMM_TOPK_CASE(9) TGMM_TOPK_CASE(10) TGMM_TOPK_CASE(11)
+      TGMM_TOPK_CASE(1) TGMM_TOPK_CASE(2) TGMM_TOPK_CASE(3) TGMM_TOPK_CASE(4) TGMM_TOPK_CASE(5) TGMM_TOPK_CASE(6)
+      TGMM_TOPK_CASE(7) TGMM_TOPK_CASE(8) TGMM_TOPK_CASE(9) TGMM_TOPK_CASE(10) TGMM_TOPK_CASE(11)
 #undef TGMM_TOPK_CASE
-    default:
-      break;
+      default:
+        break;
+    }
+    e = cudaGetLastError();
   }
-  e = cudaGetLastError();
-  cudaFreeAsync(buf, st);
-  return e;
-}
-
-// Bytes of scratch the grid kNN needs for nref reference points.
-size_t knn_grid_scratch_bytes(int32_t nref) {
-  const size_t budget = 2 * (size_t)nref + 2;
-  const size_t refs_off = (256 + 4 * budget + 4 * (budget + 1) + 4 * budget + 4 * (size_t)nref + 255) / 256 * 256;
-  return refs_off + 16 * (size_t)nref;
+  const cudaError_t ef = cudaFreeAsync(buf, st);
+  return e != cudaSuccess ? e : ef;
 }
 
 // The grid kNN on caller-provided scratch (at least knn_grid_scratch_bytes(nref), 256-byte
 // aligned); allocates nothing.
 cudaError_t knn_grid_in_scratch(const float* q, int64_t nq, const float* ref, int32_t nref, const float scale[3],
                                 int32_t* ind, cudaStream_t st, void* scratch) {
-  const int budget = 2 * nref + 2;
-  char* buf = (char*)scratch;
-  const size_t off_state = 0, off_cnt = 256, off_start = off_cnt + 4 * (size_t)budget,
-               off_cur = off_start + 4 * ((size_t)budget + 1), off_rc = off_cur + 4 * (size_t)budget,
-               off_refs = (off_rc + 4 * (size_t)nref + 255) / 256 * 256;
-  static_assert(sizeof(FrameState) <= 256, "the grid geometry record fits the scratch's 256-byte header");
-  FrameState* S = (FrameState*)(buf + off_state);
-  int* cnt = (int*)(buf + off_cnt);
-  int* start = (int*)(buf + off_start);
-  int* cur = (int*)(buf + off_cur);
-  int* rc = (int*)(buf + off_rc);
-  float4* refs = (float4*)(buf + off_refs);
-  cudaError_t e = cudaMemsetAsync(cnt, 0, 4 * (size_t)budget, st);  // counts start at zero every call
+  SaScratch w;
+  cudaError_t e = sa_build(q, nq, ref, nref, 3, 1, scale, kJ, (char*)scratch, &w, st);
   if (e != cudaSuccess) return e;
-  k_sa_geometry<<<1, 1024, 0, st>>>(q, nq, scale[0], scale[1], scale[2], nref, budget, S);
-  const int gb = (nref + 255) / 256;
-  k_sa_count<<<gb, 256, 0, st>>>(ref, nref, 3, 1, scale[0], scale[1], scale[2], S, cnt, rc);
-  k_sa_scan<<<1, 1024, 0, st>>>(S, cnt, start, cur);
-  k_sa_fill<<<gb, 256, 0, st>>>(ref, nref, 3, 1, rc, cur, refs);
-  k_sa_query<<<(unsigned)((nq + 127) / 128), 128, 0, st>>>(q, nq, ref, nref, scale[0], scale[1], scale[2], S, start,
-                                                          refs, ind);
+  sa_query<kJ, false>(q, nq, ref, nref, 3, 1, scale, w, ind, nullptr, st);
   return cudaGetLastError();
 }
 

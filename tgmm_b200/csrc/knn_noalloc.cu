@@ -18,9 +18,7 @@ namespace {
 
 // Scratch for TGMM_KNN_NOALLOC_MAX_REF reference points (about 2.8 MB on each device that
 // loads the library).
-constexpr size_t kScratchBytes = (256 + 4 * (2 * (size_t)TGMM_KNN_NOALLOC_MAX_REF + 2) * 3 + 4 +
-                                  4 * (size_t)TGMM_KNN_NOALLOC_MAX_REF + 255) / 256 * 256 +
-                                 16 * (size_t)TGMM_KNN_NOALLOC_MAX_REF;
+constexpr size_t kScratchBytes = tgmm::knn_grid_scratch_bytes(TGMM_KNN_NOALLOC_MAX_REF);
 
 static __device__ __align__(256) unsigned char g_knn_scratch[kScratchBytes];
 

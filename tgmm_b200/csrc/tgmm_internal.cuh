@@ -282,8 +282,15 @@ cudaError_t knn_grid_standalone(const float* query, int64_t nq, const float* ref
                                 int32_t nref, const float scale[3], int32_t* ind,
                                 cudaStream_t st);
 
+// Scratch of the standalone grid kNN over nref reference points: a header (grid geometry,
+// box keys), counts and first places of 2 nref + 2 cells, each reference's cell and place, the
+// references cell by cell.
+constexpr size_t kSaBox = 256, kSaClear = 512;
+constexpr size_t knn_scratch_start(size_t nref) { return kSaClear + 4 * (2 * nref + 2); }
+constexpr size_t knn_scratch_place(size_t nref) { return (knn_scratch_start(nref) + 4 * (2 * nref + 2) + 15) / 16 * 16; }
+constexpr size_t knn_scratch_refs(size_t nref) { return (knn_scratch_place(nref) + 8 * nref + 255) / 256 * 256; }
+constexpr size_t knn_grid_scratch_bytes(size_t nref) { return knn_scratch_refs(nref) + 16 * nref; }
 // grid kNN on caller-provided scratch (no allocation)
-size_t knn_grid_scratch_bytes(int32_t nref);
 constexpr int kMaxK = 11;  // neighbours of the tracking graph's supervoxel kNN (maxKNN)
 cudaError_t knn_grid_topk(const float* q, int64_t nq, const float* ref, int32_t nref, int soa, int K,
                           const float scale[3], int32_t* ind, float* dist, cudaStream_t st);
