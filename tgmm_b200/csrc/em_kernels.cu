@@ -3173,42 +3173,50 @@ cudaError_t knn_grid_in_scratch(const float* q, int64_t nq, const float* ref, in
 // Posterior -> prior on the device (GaussianMixtureModel::updatePriors,
 // GaussianMixtureModel.cpp:892-910; N_k = nu_k - nu_o as copyFromGMEM_CUDA/updateNk
 // derive it; then nu_k *= 2, W_k /= 2 as mainTrackingGaussianMixtureModel.cpp:961-969).
-// One block: the optional alpha total is a fixed-order block sum.
+// kPriorsPerBlock records a block.  The optional alpha total (alpha_k is not written here) is
+// the same fixed-order sum in every block, so no block waits for another: 8 bytes of each
+// record read again per block, against a second launch and a place for the total.  Bound by
+// latency; 5000 records: 76 us in one block, 9.4 us this way.
 // ---------------------------------------------------------------------------
+constexpr int kPriorsPerBlock = 256;
 __global__ void __launch_bounds__(1024) k_update_priors(TgmmGaussian* gm, int n, double bp, double np, double ap,
                                                         double atot, int compute) {
   __shared__ double sh[32];
-  __shared__ double s_tot;
   if (compute && atot < 0.0) {
     double a = 0.0;
-    for (int k = threadIdx.x; k < n; k += blockDim.x) a += gm[k].alpha_k;
+#pragma unroll 8
+    for (int k = threadIdx.x; k < n; k += 1024) a += gm[k].alpha_k;
     a = warp_sum(a);
     if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = a;
     __syncthreads();
-    if (threadIdx.x == 0) {
-      double t = 0.0;
-      for (int i = 0; i < (int)(blockDim.x >> 5); i++) t += sh[i];
-      s_tot = t;
-    }
-    __syncthreads();
-    atot = s_tot;
+    atot = 0.0;
+#pragma unroll
+    for (int i = 0; i < 32; i++) atot += sh[i];
   }
-  for (int k = threadIdx.x; k < n; k += blockDim.x) {
-    TgmmGaussian& g = gm[k];
-    const double Nk = g.nu_k - g.nu_o;
-    for (int d = 0; d < 3; d++) g.m_o[d] = g.m_k[d];
-    g.beta_o = fmax(bp * Nk, 1e-5);
-    g.nu_o = fmax(np * Nk, 3.0);
-    for (int e = 0; e < 6; e++) g.W_o[e] = g.W_k[e] * g.nu_k / g.nu_o;
-    if (atot >= 0.0) g.alpha_o = atot * TGMM_MIN_PI_FOR_DEAD * ap;
-    g.nu_k *= 2.0;
-    for (int e = 0; e < 6; e++) g.W_k[e] /= 2.0;
-  }
+  const int k = blockIdx.x * kPriorsPerBlock + threadIdx.x;
+  if (threadIdx.x >= kPriorsPerBlock || k >= n) return;
+  TgmmGaussian& g = gm[k];
+  const double nu = g.nu_k, Nk = nu - g.nu_o, nuo = fmax(np * Nk, 3.0);
+  double m[3], W[6];
+#pragma unroll
+  for (int d = 0; d < 3; d++) m[d] = g.m_k[d];
+#pragma unroll
+  for (int e = 0; e < 6; e++) W[e] = g.W_k[e];
+#pragma unroll
+  for (int d = 0; d < 3; d++) g.m_o[d] = m[d];
+  g.beta_o = fmax(bp * Nk, 1e-5);
+  g.nu_o = nuo;
+#pragma unroll
+  for (int e = 0; e < 6; e++) g.W_o[e] = W[e] * nu / nuo;
+  if (atot >= 0.0) g.alpha_o = atot * TGMM_MIN_PI_FOR_DEAD * ap;
+  g.nu_k = nu * 2.0;
+#pragma unroll
+  for (int e = 0; e < 6; e++) g.W_k[e] = W[e] / 2.0;
 }
 
 cudaError_t update_priors_device(TgmmGaussian* gm, int32_t n, double bp, double np, double ap, double atot,
                                  int compute, cudaStream_t st) {
-  k_update_priors<<<1, 1024, 0, st>>>(gm, n, bp, np, ap, atot, compute);
+  k_update_priors<<<(n + kPriorsPerBlock - 1) / kPriorsPerBlock, 1024, 0, st>>>(gm, n, bp, np, ap, atot, compute);
   return cudaGetLastError();
 }
 
