@@ -3122,7 +3122,7 @@ static cudaError_t sa_build(const float* q, int64_t nq, const float* ref, int32_
 cudaError_t knn_grid_standalone(const float* q, int64_t nq, const float* ref, int32_t nref, const float scale[3],
                                 int32_t* ind, cudaStream_t st) {
   char* buf = nullptr;
-  cudaError_t e = cudaMallocAsync((void**)&buf, knn_grid_scratch_bytes(nref), st);
+  cudaError_t e = scratch_alloc((void**)&buf, knn_grid_scratch_bytes(nref), st);
   if (e != cudaSuccess) return e;
   e = knn_grid_in_scratch(q, nq, ref, nref, scale, ind, st, buf);
   const cudaError_t ef = cudaFreeAsync(buf, st);
@@ -3136,7 +3136,7 @@ cudaError_t knn_grid_topk(const float* q, int64_t nq, const float* ref, int32_t 
   const int step = soa ? 1 : 3;
   const int64_t comp = soa ? nref : 1;
   char* buf = nullptr;
-  cudaError_t e = cudaMallocAsync((void**)&buf, knn_grid_scratch_bytes(nref), st);
+  cudaError_t e = scratch_alloc((void**)&buf, knn_grid_scratch_bytes(nref), st);
   if (e != cudaSuccess) return e;
   SaScratch w;
   e = sa_build(q, nq, ref, nref, step, comp, scale, K, buf, &w, st);

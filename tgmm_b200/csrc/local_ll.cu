@@ -174,7 +174,7 @@ extern "C" int tgmm_local_likelihood(const TgmmFrame* frame, const int32_t* ind_
   const size_t o_a = o_item + 8 * (size_t)(n_items > 0 ? n_items : 1);
   const size_t o_ll = o_a + 8, total = o_ll + 8 * ((size_t)n_lists + 1);
   char* buf = nullptr;
-  cudaError_t e = cudaMallocAsync((void**)&buf, total, st);
+  cudaError_t e = scratch_alloc((void**)&buf, total, st);
   if (e != cudaSuccess) return report_error(TGMM_ERR_OOM, "tgmm_local_likelihood: scratch", e);
   int32_t* d_ptr = (int32_t*)buf;
   int32_t* d_idx = d_ptr + n_lists + 1;

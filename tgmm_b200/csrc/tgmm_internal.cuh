@@ -296,6 +296,8 @@ cudaError_t knn_grid_topk(const float* q, int64_t nq, const float* ref, int32_t 
                           const float scale[3], int32_t* ind, float* dist, cudaStream_t st);
 cudaError_t knn_grid_in_scratch(const float* query, int64_t nq, const float* ref_xyz, int32_t nref,
                                 const float scale[3], int32_t* ind, cudaStream_t st, void* scratch);
+// stream-ordered scratch of one call on the current device, freed with cudaFreeAsync
+cudaError_t scratch_alloc(void** p, size_t bytes, cudaStream_t st);
 // records a failure for tgmm_last_error() and returns code
 int report_error(int code, const char* what, cudaError_t e);
 
