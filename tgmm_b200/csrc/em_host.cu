@@ -41,7 +41,7 @@ int64_t align_up(int64_t x, int64_t a) { return (x + a - 1) / a * a; }
 
 struct Layout {
   // byte offsets of every device array inside one allocation
-  int64_t info, frames, state, gchunks, g_frame, gd, fixed, cell_refs, cell_cnt, bcnt, bucket, acnt, abucket, ape, apf, dead, ec, llc, kpos, work, sv_frame, sv_order, ord_hist, ord_cur, sv_rec, sv_ll, vox4, mom, cand, rnk, nbr, nbr_b, llp, gm_scratch, total;
+  int64_t info, frames, state, gchunks, g_frame, gd, fixed, cell_refs, cell_cnt, bcnt, bucket, acnt, abucket, ape, apf, dead, ec, llc, gll, kpos, work, sv_frame, sv_order, ord_hist, ord_cur, sv_rec, sv_ll, vox4, mom, cand, rnk, nbr, nbr_b, llp, gm_scratch, total;
 };
 
 Layout make_layout(const TgmmPlanDesc& d, int32_t max_gchunks, int32_t max_cells) {
@@ -71,6 +71,7 @@ Layout make_layout(const TgmmPlanDesc& d, int32_t max_gchunks, int32_t max_cells
   L.dead = take(4 * (int64_t)max_gchunks);
   L.ec = take(8 * kEcStride * G);
   L.llc = take(8 * 10 * G);
+  L.gll = take((int64_t)sizeof(GaussLL) * G);
   L.kpos = take(16 * G);
   L.work = take(64);
   L.sv_frame = take(4 * S);
@@ -255,6 +256,7 @@ int tgmm_plan_create(const TgmmPlanDesc* d, TgmmPlan** out) {
   D.dead_part = (int32_t*)(b + P->L.dead);
   D.ec = (double*)(b + P->L.ec);
   D.llc = (double*)(b + P->L.llc);
+  D.gll = (GaussLL*)(b + P->L.gll);
   D.kpos = (float4*)(b + P->L.kpos);
   D.work = (int32_t*)(b + P->L.work);
   D.knn_group = 8;

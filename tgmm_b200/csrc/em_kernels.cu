@@ -14,6 +14,8 @@
 #include <string.h>
 
 #include <algorithm>
+#include <cstddef>
+#include <type_traits>
 
 #include "tgmm_internal.cuh"
 
@@ -232,13 +234,12 @@ __device__ void write_sv_rec(const DevPlan& P, const FrameDesc& D, int f, int s,
   l.v0 = D.vox_base + (nt ? a : 0);
   l.nv = nv;
   l.ntiles = nt;
-  l.r0 = r0;
   l.frame = f;
   l.frame_nsv = D.n_sv;
   l.c0 = r.c0;
   l.c1 = r.c1;
   l.c2 = r.c2;
-  l.pad[0] = l.pad[1] = 0;
+  l.h0 = l.h1 = l.h2 = 0.0f;  // the moment pass's
   P.sv_ll[s] = l;
 }
 
@@ -1270,6 +1271,30 @@ __global__ void __launch_bounds__(kMChunk) k_mstep_update(DevPlan P) {
   if ((threadIdx.x & 31) == 0 && mv > 0.0f) atomicMax(&P.state[ch.frame].disp_max, __float_as_uint(mv));
 }
 
+// The log-likelihood pass's record of a Gaussian (see GaussLL): Cholesky's factor of
+// nu W log2(e) / 2 from reciprocal square roots in FP64, rounded once.  Zero where the weight is
+// not finite (the candidate then counts for nothing, or rules its supervoxels out); r[0] NaN
+// where there is no factor.
+__device__ __forceinline__ GaussLL stream_record(const double* W, double nu, double ln_w, double m0, double m1,
+                                                 double m2) {
+  const double h = 0.5 * 1.4426950408889634 * nu;
+  const double i0 = rsqrt(h * W[0]);
+  const double r00 = h * W[0] * i0, r01 = h * W[1] * i0, r02 = h * W[2] * i0;
+  const double p11 = h * W[3] - r01 * r01, i1 = rsqrt(p11);
+  const double r11 = p11 * i1, r12 = (h * W[4] - r01 * r02) * i1;
+  const double p22 = h * W[5] - r02 * r02 - r12 * r12;
+  const double r22 = p22 * rsqrt(p22);
+  GaussLL g;
+  g.b = ln_w * 1.4426950408889634;
+  g.m[0] = m0, g.m[1] = m1, g.m[2] = m2;
+  const double r[6] = {r00, r01, r02, r11, r12, r22};
+  bool ok = true;
+  for (int e = 0; e < 6; e++) ok = ok && isfinite(r[e]);
+  for (int e = 0; e < 6; e++) g.r[e] = !isfinite(ln_w) ? 0.0f : ok ? __double2float_rn(r[e]) : __uint_as_float(0x7fffffffu);
+  g.pad[0] = g.pad[1] = 0.0f;
+  return g;
+}
+
 // ===========================================================================
 // kill_prep: dead-Gaussian rule (GMEMcheckDeadCellsKernel, GMEMupdateCUDA.cu:1813-1843)
 // with the post-update alpha total, then the preparation of the next iteration.
@@ -1291,13 +1316,18 @@ __global__ void __launch_bounds__(kGChunk) k_kill_prep(DevPlan P) {
   bool nanw = false, was_dead = true, fixed = true;
   double a = 0.0;
   float4 centre = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  GaussLL rec;
   if (valid) {
     centre = P.kpos[k];
     nanw = isnan(gcomp(P, G_ELD0 + cur, k));
-    for (int e = 0; e < 6; e++) nanw = nanw || isnan(gcomp(P, G_W0 + e, k));
+    double Wk[6];
+    for (int e = 0; e < 6; e++) Wk[e] = gcomp(P, G_W0 + e, k);
     a = gcomp(P, G_ALPHA, k);
     was_dead = is_dead_prior(gcomp(P, G_MO0, k));
     fixed = P.fixed[k] != 0;
+    for (int e = 0; e < 6; e++) nanw = nanw || isnan(Wk[e]);
+    rec = stream_record(Wk, gcomp(P, G_NU, k), P.llc[(int64_t)k * 10 + 6], gcomp(P, G_M0, k), gcomp(P, G_M1, k),
+                        gcomp(P, G_M2, k));
   }
   __shared__ int s_fast;
   int cell = -1;
@@ -1347,6 +1377,7 @@ __global__ void __launch_bounds__(kGChunk) k_kill_prep(DevPlan P) {
   if (s_fast) {
     // nothing dies: the live Gaussians go into the grid, and the frame's first chunk writes
     // its totals (the post-kill total is the M-step's; the dead count stays)
+    if (valid) P.gll[k] = rec;
     if (valid && !was_dead) grid_insert_at(P, D, cell, k, centre);
     if (c == D.gchunk_base && threadIdx.x == 0) {
       FrameState* Sw = &P.state[ch.frame];
@@ -1372,12 +1403,14 @@ __global__ void __launch_bounds__(kGChunk) k_kill_prep(DevPlan P) {
       const double I6[6] = {1, 0, 0, 1, 0, 1};
       for (int e = 0; e < 6; e++) gcomp(P, G_W0 + e, k) = I6[e];
       write_records(P, D, k, nxt, true, I6, gcomp(P, G_NU, k), 0.0, gcomp(P, G_BETA, k), mdead, false);
+      rec = stream_record(I6, gcomp(P, G_NU, k), -kInf, mdead[0], mdead[1], mdead[2]);
       dead = 1;
     } else {
       alpha = a;
       dead = was_dead ? 1 : 0;
       if (!was_dead) grid_insert_at(P, D, cell, k, centre);
     }
+    P.gll[k] = rec;
   }
   chunk_partials(alpha, dead, shd, shi, P.alpha_part_f, P.dead_part, c);
   chunk_done(P, ch.frame, D.n_gchunks, nxt);
@@ -1390,13 +1423,8 @@ __global__ void __launch_bounds__(kGChunk) k_kill_prep(DevPlan P) {
 // GMEMupdateCUDA.cu:1913-1978), I_v * ll_v summed when the density is positive.  Two
 // sums: every voxel (true) and the reference's per-thread overwrite for supervoxels
 // above 1024 voxels (as reference).
-// Voxels are centred at the supervoxel centroid c (e = x - c is exact in FP32 for voxels
-// near c) and candidate j enters through u_j = m_j - c, formed in FP64 and rounded once.
-// With a_j = ln weight_j - nu_j d'W_j d/2 (d = e - u_j) each voxel's term
-//   ll_v = a_max + ln sum_j exp(a_j - a_max)
-// is evaluated in FP32, the five candidates in packed FP32x2 pairs (absolute error of a
-// term about 1e-6); a lane adds its voxels of a tile in FP32 and the tile sums in FP64.
-// The FP64 mode evaluates every component in FP64 with the reference's formula.
+// k_ll_pass holds the FP64 mode (every component in FP64 with the reference's formula) and, on
+// the same tile ring, the once-per-call moment pass; the FP32 mode is k_ll_stream below.
 // Voxel tiles reach shared memory through TMA bulk copies (cp.async.bulk, one per
 // component and tile, issued by one lane) that complete on a per-slot mbarrier:
 // kLLStages tiles of kLLTile voxels are in flight per warp while it computes.  A copy
@@ -1408,7 +1436,6 @@ __global__ void __launch_bounds__(kGChunk) k_kill_prep(DevPlan P) {
 // convergence test for that frame.
 // ===========================================================================
 constexpr float kL2E = 1.4426950408889634f;  // log2(e)
-constexpr float kLN2F = 0.6931471805599453f;
 constexpr double kFracScale = 1099511627776.0;  // 2^40
 
 __device__ __forceinline__ float ex2_approx(float x) {
@@ -1420,87 +1447,6 @@ __device__ __forceinline__ float lg2_approx(float x) {
   float y;
   asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
-}
-
-// FP32 constants of the five candidates: two packed pairs and one single.
-struct CandF {
-  float2 u[2][3];
-  float2 A[2][6];
-  float2 b[2];
-  float u4[3], A4[6], b4;
-};
-
-// The candidates' constants from shared memory into a register copy; the 4-DOF form leaves the
-// W02 and W12 entries (zero there) out, so that they are not kept live.
-template <bool kW4>
-__device__ __forceinline__ CandF load_cand(const CandF& S) {
-  CandF C;
-#pragma unroll
-  for (int q = 0; q < 2; q++) {
-#pragma unroll
-    for (int d = 0; d < 3; d++) C.u[q][d] = S.u[q][d];
-#pragma unroll
-    for (int e = 0; e < 6; e++) C.A[q][e] = (kW4 && (e == 2 || e == 4)) ? make_float2(0.0f, 0.0f) : S.A[q][e];
-    C.b[q] = S.b[q];
-  }
-#pragma unroll
-  for (int d = 0; d < 3; d++) C.u4[d] = S.u4[d];
-#pragma unroll
-  for (int e = 0; e < 6; e++) C.A4[e] = (kW4 && (e == 2 || e == 4)) ? 0.0f : S.A4[e];
-  C.b4 = S.b4;
-  return C;
-}
-
-template <bool kW4>
-__device__ __forceinline__ float2 eval_pair(const CandF& C, int q, float2 E0, float2 E1, float2 E2) {
-  const float2 d0 = __fadd2_rn(E0, C.u[q][0]);  // u stored negated
-  const float2 d1 = __fadd2_rn(E1, C.u[q][1]);
-  const float2 d2 = __fadd2_rn(E2, C.u[q][2]);
-  const float2* A = C.A[q];
-  if (kW4) {
-    const float2 t0 = __ffma2_rn(A[1], d1, __fmul2_rn(A[0], d0));
-    return __ffma2_rn(d0, t0, __ffma2_rn(d1, __fmul2_rn(A[3], d1), __ffma2_rn(d2, __fmul2_rn(A[5], d2), C.b[q])));
-  } else {
-    const float2 t0 = __ffma2_rn(A[0], d0, __ffma2_rn(A[1], d1, __fmul2_rn(A[2], d2)));
-    const float2 t1 = __ffma2_rn(A[3], d1, __fmul2_rn(A[4], d2));
-    return __ffma2_rn(d0, t0, __ffma2_rn(d1, t1, __ffma2_rn(d2, __fmul2_rn(A[5], d2), C.b[q])));
-  }
-}
-
-template <bool kW4>
-__device__ __forceinline__ float eval_single(const CandF& C, float e0, float e1, float e2) {
-  const float d0 = e0 + C.u4[0], d1 = e1 + C.u4[1], d2 = e2 + C.u4[2];
-  const float* A = C.A4;
-  if (kW4) {
-    const float t0 = fmaf(A[1], d1, A[0] * d0);
-    return fmaf(d0, t0, fmaf(d1, A[3] * d1, fmaf(d2, A[5] * d2, C.b4)));
-  } else {
-    const float t0 = fmaf(A[0], d0, fmaf(A[1], d1, A[2] * d2));
-    const float t1 = fmaf(A[3], d1, A[4] * d2);
-    return fmaf(d0, t0, fmaf(d1, t1, fmaf(d2, A[5] * d2, C.b4)));
-  }
-}
-
-// max of three (one instruction on sm_100; the NaN rule of fmaxf: a NaN operand is ignored)
-__device__ __forceinline__ float fmax3(float a, float b, float c) {
-  float r;
-  asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
-  return r;
-}
-
-template <bool kW4>
-__device__ __forceinline__ float voxel_ll_f32(const CandF& C, float e0, float e1, float e2) {
-  const float2 E0 = make_float2(e0, e0), E1 = make_float2(e1, e1), E2 = make_float2(e2, e2);
-  const float2 a01 = eval_pair<kW4>(C, 0, E0, E1, E2);
-  const float2 a23 = eval_pair<kW4>(C, 1, E0, E1, E2);
-  const float a4 = eval_single<kW4>(C, e0, e1, e2);
-  const float am = fmax3(fmax3(a01.x, a01.y, a23.x), a23.y, a4);
-  const float nm = -am * kL2E;
-  const float2 t01 = __ffma2_rn(a01, make_float2(kL2E, kL2E), make_float2(nm, nm));
-  const float2 t23 = __ffma2_rn(a23, make_float2(kL2E, kL2E), make_float2(nm, nm));
-  const float s = (ex2_approx(t01.x) + ex2_approx(t01.y)) + (ex2_approx(t23.x) + ex2_approx(t23.y)) +
-                  ex2_approx(fmaf(a4, kL2E, nm));
-  return fmaf(lg2_approx(s), kLN2F, am);
 }
 
 // FP64 verification mode: the reference's formula, every component in FP64.
@@ -1650,10 +1596,9 @@ static_assert(sizeof(LLRec) % 16 == 0 && sizeof(LLConst) % 16 == 0, "look-ahead 
 constexpr int kLLBarOff = kLLStages * kLLSlotFloats * 4;
 constexpr int kLLRecOff = (kLLBarOff + kLLStages * 8 + 15) / 16 * 16;
 constexpr int kLLConstOff = kLLRecOff + 3 * (int)sizeof(LLRec);
-constexpr int kLLCandOff = kLLConstOff + 2 * (int)sizeof(LLConst);
-constexpr int kLLWarpBytes = (kLLCandOff + (int)sizeof(CandF) + 15) / 16 * 16;
+constexpr int kLLWarpBytes = (kLLConstOff + 2 * (int)sizeof(LLConst) + 15) / 16 * 16;
 constexpr size_t kLLSmemBytes = (size_t)kLLWarpBytes * kLLWarps;
-static_assert((kLLSlotFloats * 4) % 16 == 0 && kLLRecOff % 16 == 0 && kLLConstOff % 16 == 0 && kLLCandOff % 16 == 0,
+static_assert((kLLSlotFloats * 4) % 16 == 0 && kLLRecOff % 16 == 0 && kLLConstOff % 16 == 0,
               "slots and records stay 16-byte aligned");
 // the FP32 forms keep kLLBlocks blocks on an SM (228 KB of shared memory, 1 KB reserved per
 // block, the FP32 forms' one static LLShared64); the FP64 form sizes its own grid
@@ -1690,30 +1635,8 @@ __device__ __forceinline__ void ll_fetch_b(const DevPlan& P, const LLRec& A, int
   }
 }
 
-// Tile t of a supervoxel from the centred voxel stream: one bulk copy of its float4 voxels
-// (16 bytes each, so every tile starts and ends on a 16-byte boundary).
-__device__ __forceinline__ void ll_issue4(const float4* vox4, const SvLL& R, int t, float* slot, unsigned bar) {
-  const int off = t == 0 ? 0 : R.r0 + kLLTile * (t - 1);
-  const unsigned bytes = 16u * (unsigned)(t == 0 ? R.r0 : kLLTile);
-  mbar_expect_tx(bar, bytes);
-  bulk_g2s(smem_addr(slot), (unsigned long long)(vox4 + R.v0 + off), bytes, bar);
-}
-
-// Evaluation of one voxel in the three modes: 0 FP32 4-DOF, 1 FP32 general, 2 FP64.
-template <int kMode>
-struct VoxelEval {
-  using T = float;
-  const CandF& C;
-  __device__ __forceinline__ float operator()(float x, float y, float z, float c0, float c1, float c2) const {
-    return voxel_ll_f32<kMode == 0>(C, x - c0, y - c1, z - c2);
-  }
-  // from e = x - c as the moment pass stored it (the same FP32 value as x - c0 above)
-  __device__ __forceinline__ float e(float e0, float e1, float e2) const { return voxel_ll_f32<kMode == 0>(C, e0, e1, e2); }
-  __device__ __forceinline__ static bool ok(float l) { return l > -745.13f; }  // exp(l) is a positive double
-};
-template <>
-struct VoxelEval<2> {
-  using T = double;
+// Evaluation of one voxel in FP64.
+struct VoxelEval64 {
   const LLShared64& C;
   __device__ __forceinline__ double operator()(float x, float y, float z, float c0, float c1, float c2) const {
     bool ok;
@@ -1726,10 +1649,9 @@ struct VoxelEval<2> {
 // One staged tile: lane voxels o = u*32 + lane, sht[c] the offset of component c in the
 // slot.  kFull: all kLLTile voxels present (else the first rem).  allok turns false when
 // a present voxel has a zero density.
-template <class Eval, bool kFull>
-__device__ __forceinline__ void ll_tile(const Eval& eval, const float* __restrict__ slot, const int* sht, int rem,
-                                        float c0, float c1, float c2, typename Eval::T& tsum, bool& allok) {
-  using T = typename Eval::T;
+template <bool kFull>
+__device__ __forceinline__ void ll_tile(const VoxelEval64& eval, const float* __restrict__ slot, const int* sht, int rem,
+                                        float c0, float c1, float c2, double& tsum, bool& allok) {
   const int lane = threadIdx.x & 31;
   const float* bx = slot + sht[0] + lane;
   const float* by = slot + kLLSpan + sht[1] + lane;
@@ -1738,43 +1660,24 @@ __device__ __forceinline__ void ll_tile(const Eval& eval, const float* __restric
 #pragma unroll
   for (int u = 0; u < kLLTile / 32; u++) {
     if (!kFull && u * 32 >= rem) break;
-    const T l = eval(bx[32 * u], by[32 * u], bz[32 * u], c0, c1, c2);
-    const bool ok = Eval::ok(l);
+    const double l = eval(bx[32 * u], by[32 * u], bz[32 * u], c0, c1, c2);
+    const bool ok = VoxelEval64::ok(l);
     const bool in = kFull || u * 32 + lane < rem;
     allok = allok && (ok || !in);
-    tsum += (in && ok) ? (T)bi[32 * u] * l : (T)0;
-  }
-}
-
-// The same tile from the centred voxel stream: lane voxels o = u*32 + lane, each one float4
-// (e0, e1, e2, I) read with one shared-memory load.
-template <class Eval, bool kFull>
-__device__ __forceinline__ void ll_tile4(const Eval& eval, const float4* __restrict__ slot, int rem, float& tsum,
-                                         bool& allok) {
-  const int lane = threadIdx.x & 31;
-#pragma unroll
-  for (int u = 0; u < kLLTile / 32; u++) {
-    if (!kFull && u * 32 >= rem) break;
-    const float4 v = slot[32 * u + lane];
-    const float l = eval.e(v.x, v.y, v.z);
-    const bool ok = Eval::ok(l);
-    const bool in = kFull || u * 32 + lane < rem;
-    allok = allok && (ok || !in);
-    tsum += (in && ok) ? v.w * l : 0.0f;
+    tsum += (in && ok) ? (double)bi[32 * u] * l : 0.0;
   }
 }
 
 // A kept voxel (one of the last 1024 of a supervoxel above 1024 voxels) with a zero
 // density: the reference thread of its stride still holds the last voxel of the stride
 // with a positive density (GMEMupdateCUDA.cu:1961-1962).  Rare; reads global memory.
-template <class Eval>
-__device__ __forceinline__ double ll_walk_back(const Eval& eval, const SvRec& R, int i, float c0, float c1, float c2) {
+__device__ __forceinline__ double ll_walk_back(const VoxelEval64& eval, const SvRec& R, int i, float c0, float c1, float c2) {
   const float* v[4];
 #pragma unroll
   for (int c = 0; c < 4; c++) v[c] = reinterpret_cast<const float*>(R.lo0[c]) + ((R.nf[c] >> 16) & 3);
   for (int i2 = i - 1024; i2 >= 0; i2 -= 1024) {
-    const typename Eval::T l2 = eval(v[0][i2], v[1][i2], v[2][i2], c0, c1, c2);
-    if (Eval::ok(l2)) return (double)v[3][i2] * (double)l2;
+    const double l2 = eval(v[0][i2], v[1][i2], v[2][i2], c0, c1, c2);
+    if (VoxelEval64::ok(l2)) return (double)v[3][i2] * (double)l2;
   }
   return 0.0;
 }
@@ -1782,8 +1685,7 @@ __device__ __forceinline__ double ll_walk_back(const Eval& eval, const SvRec& R,
 // The kept tiles (bit t - (nt - kKeptTiles) of `mask`) that hold voxels of zero density, after the
 // supervoxel's tiles: their voxels are read again from global memory and each one of zero
 // density adds the walk-back value.  Rare.
-template <class Eval>
-__device__ __forceinline__ double ll_fixup(const Eval& eval, const SvRec& R, unsigned mask, float c0, float c1,
+__device__ __forceinline__ double ll_fixup(const VoxelEval64& eval, const SvRec& R, unsigned mask, float c0, float c1,
                                            float c2) {
   const int lane = threadIdx.x & 31;
   const float* v[4];
@@ -1797,37 +1699,8 @@ __device__ __forceinline__ double ll_fixup(const Eval& eval, const SvRec& R, uns
     const int rem = t == 0 ? R.r0 : kLLTile;
     for (int o = lane; o < rem; o += 32) {
       const int i = start + o;
-      const typename Eval::T l = eval(v[0][i], v[1][i], v[2][i], c0, c1, c2);
-      if (!Eval::ok(l)) add += ll_walk_back(eval, R, i, c0, c1, c2);
-    }
-  }
-  return add;
-}
-
-// The centred-stream forms of ll_walk_back and ll_fixup: v = the supervoxel's voxels in vox4.
-template <class Eval>
-__device__ __forceinline__ double ll_walk_back4(const Eval& eval, const float4* v, int i) {
-  for (int i2 = i - 1024; i2 >= 0; i2 -= 1024) {
-    const float4 x = v[i2];
-    const float l2 = eval.e(x.x, x.y, x.z);
-    if (Eval::ok(l2)) return (double)x.w * (double)l2;
-  }
-  return 0.0;
-}
-
-template <class Eval>
-__device__ __forceinline__ double ll_fixup4(const Eval& eval, const float4* v, int nt, int r0, unsigned mask) {
-  const int lane = threadIdx.x & 31;
-  double add = 0.0;
-  for (int k = 0; k < kKeptTiles; k++) {
-    if (!(mask & (1u << k))) continue;
-    const int t = nt - kKeptTiles + k;
-    const int start = t == 0 ? 0 : r0 + (t - 1) * kLLTile;
-    const int rem = t == 0 ? r0 : kLLTile;
-    for (int o = lane; o < rem; o += 32) {
-      const int i = start + o;
-      const float4 x = v[i];
-      if (!Eval::ok(eval.e(x.x, x.y, x.z))) add += ll_walk_back4(eval, v, i);
+      const double l = eval(v[0][i], v[1][i], v[2][i], c0, c1, c2);
+      if (!VoxelEval64::ok(l)) add += ll_walk_back(eval, R, i, c0, c1, c2);
     }
   }
   return add;
@@ -1839,7 +1712,7 @@ __device__ __forceinline__ double ll_fixup4(const Eval& eval, const float4* v, i
 // turns true on a NaN coordinate or intensity.
 template <bool kFull>
 __device__ __forceinline__ void mom_tile(const float* __restrict__ slot, const int* sht, int rem, float c0, float c1,
-                                         float c2, double* m, bool& nan_seen, float4* __restrict__ out) {
+                                         float c2, double* m, float* h, bool& nan_seen, float4* __restrict__ out) {
   const int lane = threadIdx.x & 31;
   const float* bx = slot + sht[0] + lane;
   const float* by = slot + kLLSpan + sht[1] + lane;
@@ -1853,6 +1726,9 @@ __device__ __forceinline__ void mom_tile(const float* __restrict__ slot, const i
     nan_seen |= isnan(x) || isnan(y) || isnan(z) || isnan(I);
     const float e0f = x - c0, e1f = y - c1, e2f = z - c2;
     out[32 * u + lane] = make_float4(e0f, e1f, e2f, I);
+    h[0] = fmaxf(h[0], fabsf(e0f));
+    h[1] = fmaxf(h[1], fabsf(e1f));
+    h[2] = fmaxf(h[2], fabsf(e2f));
     const double e0 = (double)e0f, e1 = (double)e1f, e2 = (double)e2f;
     const double wI = (double)I;
     m[M_E0] += e0;
@@ -1879,83 +1755,35 @@ __device__ __forceinline__ void mom_tile(const float* __restrict__ slot, const i
 }
 
 __device__ __forceinline__ void mom_consume(const float* slot, const int* pk, int t, int r0, float c0, float c1,
-                                            float c2, double* m, bool& nan_seen, float4* sv_out) {
+                                            float c2, double* m, float* h, bool& nan_seen, float4* sv_out) {
   const int sft = t == 0 ? 0 : 4;
   const int sht[4] = {(pk[0] >> sft) & 3, (pk[1] >> sft) & 3, (pk[2] >> sft) & 3, (pk[3] >> sft) & 3};
   const int rem = t == 0 ? r0 : kLLTile;
   float4* out = sv_out + (t == 0 ? 0 : r0 + kLLTile * (t - 1));
   if (rem == kLLTile)
-    mom_tile<true>(slot, sht, rem, c0, c1, c2, m, nan_seen, out);
+    mom_tile<true>(slot, sht, rem, c0, c1, c2, m, h, nan_seen, out);
   else
-    mom_tile<false>(slot, sht, rem, c0, c1, c2, m, nan_seen, out);
+    mom_tile<false>(slot, sht, rem, c0, c1, c2, m, h, nan_seen, out);
 }
 
 // Tile t (landed in `slot`) of the current supervoxel: its sum goes to lt, and to lr when
 // the tile is one of the last kKeptTiles (the reference's kept window of 1024 voxels).  A kept
 // tile of a supervoxel above 1024 voxels with a voxel of zero density is marked in fix.
-template <class Eval>
-__device__ __forceinline__ void ll_consume(const Eval& eval, const float* slot, const int* pk, int t, int nt, int nv,
+__device__ __forceinline__ void ll_consume(const VoxelEval64& eval, const float* slot, const int* pk, int t, int nt, int nv,
                                            int r0, float c0, float c1, float c2, double& lt, double& lr,
                                            unsigned& fix) {
-  using T = typename Eval::T;
   const int sft = t == 0 ? 0 : 4;
   const int sht[4] = {(pk[0] >> sft) & 3, (pk[1] >> sft) & 3, (pk[2] >> sft) & 3, (pk[3] >> sft) & 3};
   const int rem = t == 0 ? r0 : kLLTile;
-  T tsum = (T)0;
+  double tsum = 0.0;
   bool allok = true;
   if (rem == kLLTile)
-    ll_tile<Eval, true>(eval, slot, sht, rem, c0, c1, c2, tsum, allok);
+    ll_tile<true>(eval, slot, sht, rem, c0, c1, c2, tsum, allok);
   else
-    ll_tile<Eval, false>(eval, slot, sht, rem, c0, c1, c2, tsum, allok);
-  lt += (double)tsum;
+    ll_tile<false>(eval, slot, sht, rem, c0, c1, c2, tsum, allok);
+  lt += tsum;
   if (t >= nt - kKeptTiles) {
-    lr += (double)tsum;
-    if (nv > 1024 && __any_sync(0xffffffffu, !allok)) fix |= 1u << (t - (nt - kKeptTiles));
-  }
-}
-
-// A full tile without the per-voxel zero-density test: every voxel's term is added and the
-// smallest term kept; a density is zero (the reference skips such a voxel) only when a term
-// is at or below ln of the smallest double (-745.13) or NaN, and then -- rarely -- the tile
-// is evaluated again with the per-voxel test.
-template <class Eval>
-__device__ __forceinline__ void ll_tile4_full(const Eval& eval, const float4* __restrict__ slot, float& tsum,
-                                              bool& allok) {
-  const int lane = threadIdx.x & 31;
-  float s = 0.0f, lmin = kInfF;
-#pragma unroll
-  for (int u = 0; u < kLLTile / 32; u++) {
-    const float4 v = slot[32 * u + lane];
-    const float l = eval.e(v.x, v.y, v.z);
-    lmin = fminf(lmin, l);
-    s = fmaf(v.w, l, s);
-  }
-  if (__any_sync(0xffffffffu, !(lmin > -745.13f) || isnan(s))) {
-    float t = 0.0f;
-    bool ok = true;
-    ll_tile4<Eval, true>(eval, slot, kLLTile, t, ok);
-    tsum += t;
-    allok = allok && ok;
-  } else {
-    tsum += s;
-  }
-}
-
-// The centred-stream form of ll_consume (FP32 terms).
-template <class Eval>
-__device__ __forceinline__ void ll_consume4(const Eval& eval, const float* slot, int t, int nt, int nv, int r0,
-                                            double& lt, double& lr, unsigned& fix) {
-  const float4* s4 = reinterpret_cast<const float4*>(slot);
-  const int rem = t == 0 ? r0 : kLLTile;
-  float tsum = 0.0f;
-  bool allok = true;
-  if (rem == kLLTile)
-    ll_tile4_full<Eval>(eval, s4, tsum, allok);
-  else
-    ll_tile4<Eval, false>(eval, s4, rem, tsum, allok);
-  lt += (double)tsum;
-  if (t >= nt - kKeptTiles) {
-    lr += (double)tsum;
+    lr += tsum;
     if (nv > 1024 && __any_sync(0xffffffffu, !allok)) fix |= 1u << (t - (nt - kKeptTiles));
   }
 }
@@ -2007,19 +1835,11 @@ __device__ void frame_converge(const DevPlan& P, int f) {
 // earlier.  A warp adds its supervoxels' sums into fixed-point registers and publishes
 // them (with the count of supervoxels) when its frame changes and when it leaves; the
 // warp that completes a frame's count runs the convergence test.
-// With G > 0 the warps also run the kNN/E-step of the next iteration (G lanes per
-// supervoxel, 32/G supervoxels an item, from a second work counter): one item after each
-// supervoxel's look-ahead copies are issued, and the rest once the voxel work has run out.
-// It needs only what the kill step left, and its results go to the next iteration's
-// buffers, so it runs ahead of the convergence test; a frame that converges here never
-// reads them.
-template <bool kFp64, int G, bool kMom>
+// kMom: the moment pass (which also writes the centred voxel stream); else the FP64
+// log-likelihood, which reads the input arrays too (its terms start from the exact x - c).
+template <bool kMom>
 __global__ void __launch_bounds__(kLLWarps * 32, kLLBlocks) k_ll_pass(DevPlan P) {
-  // the FP32 log-likelihood streams the centred voxel stream (one float4 per voxel, one bulk
-  // copy per tile); the moment pass reads the input arrays (and writes that stream), the FP64
-  // log-likelihood reads the input arrays too (its terms start from the exact x - c)
-  constexpr bool kAos = !kFp64 && !kMom;
-  constexpr bool kRec = !kAos, kLLr = kAos || kMom, kCand = !kMom;
+  constexpr bool kRec = true, kLLr = kMom, kCand = !kMom, kFp64 = !kMom;
   const int total = P.info->total_sv;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   __shared__ LLShared64 sh64[kFp64 ? kLLWarps : 1];
@@ -2029,7 +1849,6 @@ __global__ void __launch_bounds__(kLLWarps * 32, kLLBlocks) k_ll_pass(DevPlan P)
   const unsigned bar0 = smem_addr(wbase + kLLBarOff);
   LLRec* RA = reinterpret_cast<LLRec*>(wbase + kLLRecOff);
   LLConst* RB = reinterpret_cast<LLConst*>(wbase + kLLConstOff);
-  CandF* cs = reinterpret_cast<CandF*>(wbase + kLLCandOff);
   if (lane == 0)
     for (int q = 0; q < kLLStages; q++) mbar_init(bar0 + 8 * q, 1);
   mbar_fence_init();
@@ -2074,7 +1893,7 @@ __global__ void __launch_bounds__(kLLWarps * 32, kLLBlocks) k_ll_pass(DevPlan P)
   if (lane == 0 && sc < total) tk = take();
   int sn = sc < total ? __shfl_sync(0xffffffffu, tk, 0) : total;
   if (lane == 0 && sn < total) tk = take();
-  auto frame_of = [](const LLRec& A) { return kAos ? A.ll.frame : A.rec.frame; };
+  auto frame_of = [](const LLRec& A) { return A.rec.frame; };
   if (sc < total) {
     ll_fetch_a<kRec, kLLr, kCand>(P, RA[0], sc);
     if (sn < total) ll_fetch_a<kRec, kLLr, kCand>(P, RA[1], sn);
@@ -2084,25 +1903,6 @@ __global__ void __launch_bounds__(kLLWarps * 32, kLLBlocks) k_ll_pass(DevPlan P)
     if (!kMom) ll_fetch_b(P, RA[0], frame_of(RA[0]), RB[0]);
     cp_commit();
   }
-  // the next iteration's kNN/E-step items
-  constexpr int kPerItem = G > 0 ? 32 / G : 1;
-  const int knn_items = G > 0 ? (total + kPerItem - 1) / kPerItem : 0;
-  bool knn_more = G > 0;
-  auto knn_step = [&]() {
-    if constexpr (G > 0) {
-      int item = 0;
-      if (lane == 0) item = atomicAdd(&P.work[2], 1);
-      item = __shfl_sync(0xffffffffu, item, 0);
-      if (item < knn_items) {
-        const int gl = lane & (G - 1), gbase = lane - gl;
-        const unsigned gmask = G == 32 ? 0xffffffffu : ((1u << G) - 1u) << gbase;
-        knn_estep_sv<G>(P, item * kPerItem + gbase / G, P.iter + 1, gl, gbase, gmask);
-        __syncwarp();
-      } else {
-        knn_more = false;
-      }
-    }
-  };
   for (unsigned i = 0; sc < total; i++) {
     // everything fetched so far was issued at least a supervoxel ago
     cp_wait_all();
@@ -2115,19 +1915,18 @@ __global__ void __launch_bounds__(kLLWarps * 32, kLLBlocks) k_ll_pass(DevPlan P)
     if (!kMom && sn < total) ll_fetch_b(P, NA, frame_of(NA), RB[(i + 1) & 1]);
     if (s2 < total) ll_fetch_a<kRec, kLLr, kCand>(P, RA[(i + 2) % 3], s2);
     cp_commit();
-    if (knn_more) knn_step();  // while this supervoxel's tiles and records land
     int in = 0;
-    const int n_nt = sn < total ? (kAos ? NA.ll.ntiles : NA.rec.ntiles) : 0;  // the next one's tiles may start early
-    const int nv = kAos ? CA.ll.nv : CA.rec.nv, nt = kAos ? CA.ll.ntiles : CA.rec.ntiles;
-    const int f = frame_of(CA), nsv = kAos ? CA.ll.frame_nsv : CA.rec.frame_nsv;
-    const float c0 = kAos ? CA.ll.c0 : CA.rec.c0, c1 = kAos ? CA.ll.c1 : CA.rec.c1, c2 = kAos ? CA.ll.c2 : CA.rec.c2;
+    const int n_nt = sn < total ? NA.rec.ntiles : 0;  // the next one's tiles may start early
+    const int nv = CA.rec.nv, nt = CA.rec.ntiles;
+    const int f = frame_of(CA), nsv = CA.rec.frame_nsv;
+    const float c0 = CA.rec.c0, c1 = CA.rec.c1, c2 = CA.rec.c2;
     S = &P.state[f];
     int pk[4] = {0, 0, 0, 0};  // SoA slot offsets of the components: tile 0 in bits 0-1, later tiles in bits 4-5
     if constexpr (kRec) {
 #pragma unroll
       for (int c = 0; c < 4; c++) pk[c] = (int)(CA.rec.nf[c] >> 16);
     }
-    const int r0 = kAos ? CA.ll.r0 : CA.rec.r0;
+    const int r0 = CA.rec.r0;
     // the next staged tile of the supervoxel (of ntr): the ring is refilled first, with the
     // current supervoxel's tiles and then the next one's; nullptr if the tile never arrived
     auto ring_next = [&](int ntr) -> const float* {
@@ -2138,10 +1937,7 @@ __global__ void __launch_bounds__(kLLWarps * 32, kLLBlocks) k_ll_pass(DevPlan P)
         const int tt = mine ? ic++ : in++;
         if (lane == 0) {
           const unsigned q = gi % kLLStages;
-          if constexpr (kAos)
-            ll_issue4(P.vox4, mine ? CA.ll : NA.ll, tt, wbuf + q * kLLSlotFloats, bar0 + 8 * q);
-          else
-            ll_issue(mine ? CA.rec : NA.rec, tt, wbuf + q * kLLSlotFloats, bar0 + 8 * q);
+          ll_issue(mine ? CA.rec : NA.rec, tt, wbuf + q * kLLSlotFloats, bar0 + 8 * q);
         }
         gi++;
       }
@@ -2154,6 +1950,7 @@ __global__ void __launch_bounds__(kLLWarps * 32, kLLBlocks) k_ll_pass(DevPlan P)
       double m[kNumMoments];
 #pragma unroll
       for (int j = 0; j < kNumMoments; j++) m[j] = 0.0;
+      float h[3] = {0.0f, 0.0f, 0.0f};  // the largest |e| along each axis
       bool nan_seen = false;
       for (int t = 0; t < nt; t++) {
         const float* slot = ring_next(nt);
@@ -2161,11 +1958,16 @@ __global__ void __launch_bounds__(kLLWarps * 32, kLLBlocks) k_ll_pass(DevPlan P)
           failed = true;
           break;
         }
-        mom_consume(slot, pk, t, r0, c0, c1, c2, m, nan_seen, P.vox4 + CA.ll.v0);
+        mom_consume(slot, pk, t, r0, c0, c1, c2, m, h, nan_seen, P.vox4 + CA.ll.v0);
         gc++;
       }
       if (failed) break;
       if (__any_sync(0xffffffffu, nan_seen) && lane == 0) atomicOr(&S->flags, F_NAN_INPUT);
+#pragma unroll
+      for (int d = 0; d < 3; d++) {
+        h[d] = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(h[d])));
+        if (lane == d) (&P.sv_ll[sc].h0)[d] = h[d];
+      }
 #pragma unroll
       for (int j = 0; j < kNumMoments; j++) m[j] = warp_sum(m[j]);
 #pragma unroll
@@ -2185,68 +1987,32 @@ __global__ void __launch_bounds__(kLLWarps * 32, kLLBlocks) k_ll_pass(DevPlan P)
     }
     const unsigned fin = __ballot_sync(0xffffffffu, lane < kJ && isfinite(b));
     const unsigned nan_w = __ballot_sync(0xffffffffu, lane < kJ && (isnan(b) || b == (double)kInfF));
-    const unsigned w4m = __ballot_sync(0xffffffffu, lane >= kJ || (h[2] == 0.0 && h[4] == 0.0));
     // a NaN weight makes the reference's density NaN for every voxel (skipped); no finite
     // weight means a zero density everywhere: the tiles are consumed unread
     const bool compute = run && fin && !nan_w;
-    if (kFp64) {
-      LLShared64& Q = sh64[warp];
-      if (lane < kJ) {
-        for (int d = 0; d < 3; d++) Q.u[lane][d] = u[d];
-        for (int e = 0; e < 6; e++) Q.A[lane][e] = (e == 0 || e == 3 || e == 5) ? -2.0 * h[e] : -h[e];
-        Q.w[lane] = exp(b);
-      }
-    } else if (lane < kJ) {
-      // the five candidates' FP32 constants in the packed layout (pairs 0-1, 2-3; single 4)
-      float* fu = lane < 4 ? &cs->u[lane >> 1][0].x + (lane & 1) : cs->u4;
-      float* fa = lane < 4 ? &cs->A[lane >> 1][0].x + (lane & 1) : cs->A4;
-      const int st = lane < 4 ? 2 : 1;
-      for (int d = 0; d < 3; d++) fu[st * d] = -__double2float_rn(u[d]);
-      for (int e = 0; e < 6; e++) fa[st * e] = __double2float_rn(h[e]);
-      if (lane < 4)
-        (&cs->b[lane >> 1].x)[lane & 1] = __double2float_rn(b);
-      else
-        cs->b4 = __double2float_rn(b);
+    LLShared64& Q = sh64[warp];
+    if (lane < kJ) {
+      for (int d = 0; d < 3; d++) Q.u[lane][d] = u[d];
+      for (int e = 0; e < 6; e++) Q.A[lane][e] = (e == 0 || e == 3 || e == 5) ? -2.0 * h[e] : -h[e];
+      Q.w[lane] = exp(b);
     }
     __syncwarp();
     double lt = 0.0, lr = 0.0;
     unsigned fix = 0;  // kept tiles with voxels of zero density
     // a finished frame issues no more tiles; those issued early are consumed unread
     const int ntr = run ? nt : ic;
-    // the supervoxel's tiles and, rarely, the kept window's zero-density voxels, with the
-    // candidates' constants of one evaluation form held in registers through the loop (the
-    // 4-DOF form keeps 40 floats live, the general one 50)
-    auto run_tiles = [&](const auto& eval) {
-      for (int t = 0; t < ntr; t++) {
-        const float* slot = ring_next(ntr);
-        if (!slot) {
-          failed = true;
-          break;
-        }
-        if (compute) {
-          if constexpr (kFp64)
-            ll_consume(eval, slot, pk, t, nt, nv, r0, c0, c1, c2, lt, lr, fix);
-          else
-            ll_consume4(eval, slot, t, nt, nv, r0, lt, lr, fix);
-        }
-        gc++;
+    // the supervoxel's tiles and, rarely, the kept window's zero-density voxels
+    const VoxelEval64 eval{Q};
+    for (int t = 0; t < ntr; t++) {
+      const float* slot = ring_next(ntr);
+      if (!slot) {
+        failed = true;
+        break;
       }
-      if (!failed && fix) {
-        if constexpr (kFp64)
-          lr += ll_fixup(eval, CA.rec, fix, c0, c1, c2);
-        else
-          lr += ll_fixup4(eval, P.vox4 + CA.ll.v0, nt, r0, fix);
-      }
-    };
-    if constexpr (kFp64) {
-      run_tiles(VoxelEval<2>{sh64[warp]});
-    } else if (w4m == 0xffffffffu) {
-      const CandF cf = load_cand<true>(*cs);
-      run_tiles(VoxelEval<0>{cf});
-    } else {
-      const CandF cf = load_cand<false>(*cs);
-      run_tiles(VoxelEval<1>{cf});
+      if (compute) ll_consume(eval, slot, pk, t, nt, nv, r0, c0, c1, c2, lt, lr, fix);
+      gc++;
     }
+    if (!failed && fix) lr += ll_fixup(eval, CA.rec, fix, c0, c1, c2);
     if (failed) break;
     if (run) {
       lt = warp_sum(lt);
@@ -2277,8 +2043,606 @@ __global__ void __launch_bounds__(kLLWarps * 32, kLLBlocks) k_ll_pass(DevPlan P)
   }
   cp_wait_all();
   publish();
-  while (knn_more) knn_step();
   if (lane == 0 && atomicAdd(&P.work[1], 1) == (int)(gridDim.x * kLLWarps) - 1) {
+    P.work[0] = 0;
+    P.work[1] = 0;
+  }
+}
+
+// ===========================================================================
+// ll_stream: the log-likelihood pass over the centred voxel stream, FP32 terms (k_ll_pass keeps
+// the moment sums and the FP64 terms).  Per voxel and candidate, with the Gaussian's record of
+// the kill step (R the upper triangle of Cholesky's factor, R'R = nu W log2(e) / 2):
+//   n_j = |R_j (e - u_j)|^2 - log2(weight_j),  ll_v = ln 2 (log2 sum_j 2^(n_min - n_j) - n_min)
+// R (e - u) = R e - k with k = R u formed in FP64 from the factor's FP32 values, so that a
+// candidate takes seven multiply-adds (4-DOF shape) and no subtraction from every voxel.
+//  - A warp's first three supervoxels come by a fixed rule, snake order over the largest-first
+//    list (warp w takes places w, 2W-1-w, 2W+w), the others by ticket, three supervoxels ahead:
+//    no ticket is waited for, and none is taken on a frame with few supervoxels.
+//  - Units of 128 voxels, each lane copying (cp.async) the very voxels it will read, so that a
+//    lane waits for its own copies only: no barrier, no elected lane.  Units are end-aligned as
+//    the tiles are; the first one's missing voxels are copied as zeros (intensity 0: they add
+//    nothing), so that one form of the loop serves every unit.
+//  - Each lane's sum over a block of four units goes into its own fixed-point pair, so that no
+//    warp reduction is left per supervoxel; lanes are added when the warp's frame changes.
+//  - Candidates that cannot come within 2^-30 of the largest term anywhere in the supervoxel's
+//    box are left out of its sums (1-Gvoxel frame: one candidate for 18% of the voxels, two for
+//    28, three 25, four 19, five 10; where nuclei crowd at one per 3000 voxels all five stay).
+// 14.5 M voxels a launch: 57.3 us, 31.0 M warp instructions (as one float4 tile ring over five
+// candidates, tickets and a warp reduction per supervoxel: 69.3 us, 40.9 M); 12.6 M voxels in 16
+// crowded volumes 67.1 -> 63.5; twelve nuclei 10.6 -> 7.1.  The stream itself takes 35 us at the
+// measured 6.5 TB/s; what is left is issue (51% of the slots; the top stall is dependent
+// instructions) at 16 warps an SM.  Measured beside it: 20 warps 59.4 / 64.0 us, 24 with a
+// shared ring of two or three 70 and more (spills), 256-voxel units 70.5, rings of 4 to 6 units
+// 61 to 70 (the L1 that the ring takes is missed), every supervoxel by rule 58.8 / 65.1, the
+// candidates' constants held in registers through the loop 61.1 / 65.5.
+// ===========================================================================
+#ifndef TGMM_LS_WARPS
+#define TGMM_LS_WARPS 4
+#endif
+#ifndef TGMM_LS_BLOCKS
+#define TGMM_LS_BLOCKS 4
+#endif
+constexpr int kLSWarps = TGMM_LS_WARPS;
+constexpr int kLSBlocks = TGMM_LS_BLOCKS;
+#ifndef TGMM_LS_RING
+#define TGMM_LS_RING 3
+#endif
+constexpr int kLSRing = TGMM_LS_RING;   // units in flight per warp
+constexpr int kLSUnit = 128;            // voxels per unit, four per lane
+constexpr int kLSFixed = 3;             // supervoxels a warp takes by rule
+constexpr int kLSKept = 1024 / kLSUnit; // units of the reference's kept window
+constexpr float kLSZero = -745.13f * kL2E;  // log2 of the smallest positive density
+// Candidates whose terms stay this many bits below the largest one over a whole supervoxel are
+// left out of its sums: at most 4 2^-30 of them, 5e-9 in log2, below the last bit of an FP32 term.
+constexpr float kLSDrop = 30.0f;
+
+// Per-warp shared region: the ring, the fixed-point sums the kept window leaves out (a pair per
+// lane), the candidates' FP32 constants, three supervoxel records with their candidate ids
+// (fetched two supervoxels ahead) and two sets of candidate records (one ahead).
+struct LSRec {
+  SvLL ll;
+  int32_t cand[8];
+};
+struct LSCand {
+  GaussLL g[kJ];
+  double ln_alpha;
+  int32_t done, pad;
+};
+struct LSWarp {
+  float4 ring[kLSRing][kLSUnit];
+  long long di[32];
+  unsigned long long dr[32];
+  float cst[56];
+  LSRec rec[3];
+  LSCand cand[2];
+};
+static_assert(sizeof(LSRec) % 16 == 0 && sizeof(LSCand) % 16 == 0 && sizeof(LSWarp) % 16 == 0 &&
+                  offsetof(LSWarp, rec) % 16 == 0 && offsetof(LSWarp, cst) % 16 == 0,
+              "copies of 16 bytes");
+constexpr size_t kLSSmemBytes = (size_t)kLSWarps * sizeof(LSWarp);
+
+// The candidates' constants in LSWarp::cst: two packed pairs (two floats a field) and a single
+// one, each r00 r01 -k0 r11 -k1 r22 -k2 -log2(weight), then r02 r12 (zero in the 4-DOF form).
+// They are read where they are used, once per unit: holding the five candidates' 40 values in
+// registers through the loop left no room for more warps (128 registers and spills at 16 warps
+// an SM).
+struct CandPair {
+  float2 r00, r01, r11, r22, k0, k1, k2, b;
+};
+__device__ __forceinline__ CandPair ls_load_pair(const float* c) {
+  const float4* p = reinterpret_cast<const float4*>(c);
+  const float4 x = p[0], y = p[1], z = p[2], w = p[3];
+  CandPair C;
+  C.r00 = make_float2(x.x, x.y), C.r01 = make_float2(x.z, x.w);
+  C.k0 = make_float2(y.x, y.y), C.r11 = make_float2(y.z, y.w);
+  C.k1 = make_float2(z.x, z.y), C.r22 = make_float2(z.z, z.w);
+  C.k2 = make_float2(w.x, w.y), C.b = make_float2(w.z, w.w);
+  return C;
+}
+// n of a pair of candidates
+__device__ __forceinline__ float2 ls_pair(const CandPair& C, const float4& v) {
+  const float2 E0 = make_float2(v.x, v.x), E1 = make_float2(v.y, v.y), E2 = make_float2(v.z, v.z);
+  const float2 s0 = __ffma2_rn(C.r00, E0, __ffma2_rn(C.r01, E1, C.k0));
+  const float2 s1 = __ffma2_rn(C.r11, E1, C.k1);
+  const float2 s2 = __ffma2_rn(C.r22, E2, C.k2);
+  return __ffma2_rn(s0, s0, __ffma2_rn(s1, s1, __ffma2_rn(s2, s2, C.b)));
+}
+// n of one candidate whose constants lie `st` floats apart
+template <bool kGeneral>
+__device__ __forceinline__ float ls_single(const float* c, int st, const float4& v) {
+  float s0 = fmaf(c[0], v.x, fmaf(c[st], v.y, c[2 * st])), s1 = fmaf(c[3 * st], v.y, c[4 * st]);
+  if (kGeneral) {
+    s0 = fmaf(c[8 * st], v.z, s0);
+    s1 = fmaf(c[9 * st], v.z, s1);
+  }
+  const float s2 = fmaf(c[5 * st], v.z, c[6 * st]);
+  return fmaf(s0, s0, fmaf(s1, s1, fmaf(s2, s2, c[7 * st])));
+}
+
+__device__ __forceinline__ float fmin3(float a, float b, float c) {
+  float r;
+  asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
+
+// log2 of the densities of kN voxels of this lane in the 4-DOF form, from the first kForm
+// candidates (of three, the third is the single one), or (kForm 0) from all five in the general
+// form.
+template <int kForm, int kN>
+__device__ __forceinline__ void ls_log2(const float* cst, const float4 (&v)[kN], float (&l)[kN]) {
+  if constexpr (kForm == 1) {
+#pragma unroll
+    for (int q = 0; q < kN; q++) l[q] = -ls_single<false>(cst, 2, v[q]);
+  } else if constexpr (kForm >= 2) {
+    float2 n0[kN], n1[kN];
+    float n4[kN];
+    {
+      const CandPair C = ls_load_pair(cst);
+#pragma unroll
+      for (int q = 0; q < kN; q++) n0[q] = ls_pair(C, v[q]);
+    }
+    if constexpr (kForm >= 4) {
+      const CandPair C = ls_load_pair(cst + 20);
+#pragma unroll
+      for (int q = 0; q < kN; q++) n1[q] = ls_pair(C, v[q]);
+    }
+    if constexpr (kForm == 3 || kForm == 5) {
+#pragma unroll
+      for (int q = 0; q < kN; q++) n4[q] = ls_single<false>(cst + 40, 1, v[q]);
+    }
+#pragma unroll
+    for (int q = 0; q < kN; q++) {
+      float nm = fminf(n0[q].x, n0[q].y);
+      if constexpr (kForm == 3) nm = fminf(nm, n4[q]);
+      if constexpr (kForm == 4) nm = fmin3(nm, n1[q].x, n1[q].y);
+      if constexpr (kForm == 5) nm = fmin3(fmin3(n0[q].x, n0[q].y, n1[q].x), n1[q].y, n4[q]);
+      float s = ex2_approx(nm - n0[q].x) + ex2_approx(nm - n0[q].y);
+      if constexpr (kForm >= 4) s += ex2_approx(nm - n1[q].x) + ex2_approx(nm - n1[q].y);
+      if constexpr (kForm == 3 || kForm == 5) s += ex2_approx(nm - n4[q]);
+      l[q] = lg2_approx(s) - nm;
+    }
+  } else {
+#pragma unroll
+    for (int q = 0; q < kN; q++) {
+      float n[kJ], s = 0.0f;
+#pragma unroll
+      for (int j = 0; j < kJ; j++) n[j] = ls_single<true>(cst + (j < 4 ? (j >> 1) * 20 + (j & 1) : 40), j < 4 ? 2 : 1, v[q]);
+      const float nm = fmin3(fmin3(n[0], n[1], n[2]), n[3], n[4]);
+#pragma unroll
+      for (int j = 0; j < kJ; j++) s += ex2_approx(nm - n[j]);
+      l[q] = lg2_approx(s) - nm;
+    }
+  }
+}
+__device__ __forceinline__ float ls_log2_one(const float* cst, float4 x) {
+  const float4 v[1] = {x};
+  float l[1];
+  ls_log2<0, 1>(cst, v, l);
+  return l[0];
+}
+
+// 16 bytes global -> shared by this lane; `bytes` 0 writes zeros and reads nothing.
+__device__ __forceinline__ void cp_async16_fill(unsigned dst, const void* src, unsigned bytes) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void cp_async16_to(unsigned dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+// Waits until at most n of this lane's groups of copies are outstanding (n >= kLSRing - 1: that
+// many).
+template <int N = kLSRing - 1>
+__device__ __forceinline__ void ls_wait(int n) {
+  if constexpr (N > 0) {
+    if (n < N) {
+      ls_wait<N - 1>(n);
+      return;
+    }
+  }
+  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+
+// A unit with the per-voxel zero-density test (the reference skips such a voxel), from its
+// place `first` on.  Rare.
+__device__ __noinline__ float ls_unit_tested(const float* cst, const float4* slot, int first, bool* allok) {
+  const int lane = threadIdx.x & 31;
+  float s = 0.0f;
+  for (int u = 0; u < kLSUnit / 32; u++) {
+    const float4 v = slot[32 * u + lane];
+    const float l = ls_log2_one(cst, v);
+    const bool ok = l > kLSZero, in = 32 * u + lane >= first;
+    *allok = *allok && (ok || !in);
+    s += (in && ok) ? v.w * l : 0.0f;
+  }
+  return s;
+}
+
+// The kept units (bit k of `mask`: unit nu - kLSKept + k) that hold voxels of zero density: the
+// reference's value for each such voxel, the last one of its stride of 1024 with a positive
+// density (in log2).  Rare; reads global memory.
+__device__ __noinline__ double ls_fixup(const float* cst, const float4* v, int nu, int r0, unsigned mask) {
+  const int lane = threadIdx.x & 31;
+  double add = 0.0;
+  for (int k = 0; k < kLSKept; k++) {
+    if (!(mask & (1u << k))) continue;
+    const int t = nu - kLSKept + k;
+    const int start = t == 0 ? 0 : r0 + (t - 1) * kLSUnit, rem = t == 0 ? r0 : kLSUnit;
+    for (int o = lane; o < rem; o += 32) {
+      const float4 x = v[start + o];
+      if (ls_log2_one(cst, x) > kLSZero) continue;
+      for (int i = start + o - 1024; i >= 0; i -= 1024) {
+        const float4 y = v[i];
+        const float l = ls_log2_one(cst, y);
+        if (l > kLSZero) {
+          add += (double)y.w * (double)l;
+          break;
+        }
+      }
+    }
+  }
+  return add;
+}
+
+// This lane's part of a unit (its slot, from the lane's own voxel on) in one of the forms: sum
+// of I log2(density), smallest log2(density).
+template <int kForm>
+__device__ __forceinline__ void ls_unit(const float* cst, const float4* slot, float& s, float& lmin) {
+  float4 v[4];
+  float l[4];
+#pragma unroll
+  for (int q = 0; q < 4; q++) v[q] = slot[32 * q];
+  ls_log2<kForm, 4>(cst, v, l);
+#pragma unroll
+  for (int q = 0; q < 4; q++) {
+    lmin = fminf(lmin, l[q]);
+    s = fmaf(v[q].w, l[q], s);
+  }
+}
+
+// A supervoxel with a candidate whose precision has no Cholesky factor (records handed in with
+// an indefinite matrix, which the regularisation never produces): every voxel from the
+// quadratic form itself in FP64.  Adds this lane's share to the two fixed-point pairs.
+__device__ __noinline__ void ls_general(const DevPlan& P, const SvLL& R, const int32_t* cand, double ln_alpha,
+                                        long long* ai, unsigned long long* ar, long long* di,
+                                        unsigned long long* dr) {
+  const int lane = threadIdx.x & 31;
+  const float4* v = P.vox4 + R.v0;
+  auto ll_of = [&](float4 x) {
+    double dens = 0.0;
+    for (int j = 0; j < kJ; j++) {
+      const double* L = P.llc + (int64_t)cand[j] * 10;
+      const double d0 = (double)x.x + ((double)R.c0 - L[7]), d1 = (double)x.y + ((double)R.c1 - L[8]),
+                   d2 = (double)x.z + ((double)R.c2 - L[9]);
+      dens += exp(L[6] - ln_alpha + L[0] * d0 * d0 + L[1] * d0 * d1 + L[2] * d0 * d2 + L[3] * d1 * d1 +
+                  L[4] * d1 * d2 + L[5] * d2 * d2);
+    }
+    return dens > 0.0 ? log(dens) : -kInf;
+  };
+  double all = 0.0, kept = 0.0;
+  for (int i = lane; i < R.nv; i += 32) {
+    const float4 x = v[i];
+    double l = ll_of(x);
+    if (l > -kInf) all += (double)x.w * l;
+    if (i < R.nv - 1024) continue;
+    double w = x.w;
+    for (int b = i - 1024; !(l > -kInf) && R.nv > 1024 && b >= 0; b -= 1024) {
+      l = ll_of(v[b]);
+      w = v[b].w;
+    }
+    if (l > -kInf) kept += w * l;
+  }
+  fixed_acc(*ai, *ar, all);
+  long long ki = 0;
+  unsigned long long kr = 0;
+  fixed_acc(ki, kr, kept);
+  long long bi = 0;
+  unsigned long long br = 0;
+  fixed_acc(bi, br, all);
+  *di += ki - bi;
+  *dr += kr - br;
+}
+
+// With G > 0 the warps also run the kNN/E-step of the next iteration (G lanes per
+// supervoxel, 32/G supervoxels an item, from a second work counter): one item after each
+// supervoxel's look-ahead copies are issued, and the rest once the voxel work has run out.
+// It needs only what the kill step left, and its results go to the next iteration's
+// buffers, so it runs ahead of the convergence test; a frame that converges here never
+// reads them.
+template <int G>
+__global__ void __launch_bounds__(kLSWarps * 32, kLSBlocks) k_ll_stream(DevPlan P) {
+  const int total = P.info->total_sv;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  // a lone frame that is done leaves nothing to do
+  if (P.info->n_frames == 1 && *(volatile const int32_t*)&P.state[0].done) return;
+  extern __shared__ __align__(128) unsigned char ll_smem[];
+  LSWarp& Sh = reinterpret_cast<LSWarp*>(ll_smem)[warp];
+  const unsigned ring_a = smem_addr(&Sh.ring[0][lane]);
+  const int W = gridDim.x * kLSWarps, w = warp * gridDim.x + blockIdx.x;
+  // the supervoxel this warp takes i-th, or -1: the first kLSFixed by rule, then by ticket
+  auto take = [&](int i) {
+    int64_t p = (int64_t)i * W + ((i & 1) ? W - 1 - w : w);
+    if (i >= kLSFixed) {
+      p = total;
+      if (total > kLSFixed * W && lane == 0) p = (int64_t)kLSFixed * W + atomicAdd(&P.work[0], 1);
+      // (lane 0's place; the others get the supervoxel where it is first used)
+    }
+    return p < total ? P.sv_order[p] : -1;
+  };
+  auto fetch_rec = [&](int s, LSRec& X) {
+    if (s < 0) return;
+    if (lane < 3)
+      cp_async16(reinterpret_cast<char*>(&X.ll) + 16 * lane, reinterpret_cast<const char*>(P.sv_ll + s) + 16 * lane);
+    else if (lane < 3 + kJ)
+      cp_async4(&X.cand[lane - 3], cand_buf(P, P.iter) + (int64_t)s * kJ + lane - 3);
+  };
+  static_assert(sizeof(GaussLL) == 64, "four lanes a candidate");
+  auto fetch_cand = [&](int s, const LSRec& A, LSCand& X) {
+    if (s < 0) return;
+    if (lane < 4 * kJ) {
+      const int j = lane >> 2;
+      cp_async16(reinterpret_cast<char*>(&X.g[j]) + 16 * (lane & 3),
+                 reinterpret_cast<const char*>(P.gll + A.cand[j]) + 16 * (lane & 3));
+    } else if (lane == 4 * kJ) {
+      cp_async8(&X.ln_alpha, &P.state[A.ll.frame].ln_alpha);
+    } else if (lane == 4 * kJ + 1) {
+      cp_async4(&X.done, &P.state[A.ll.frame].done);
+    }
+  };
+  // this lane's fixed-point sums over the warp's run of supervoxels of one frame: every voxel
+  // here, what the reference's kept window leaves out in Sh.di, Sh.dr
+  int acc_f = -1, acc_nsv = 0, acc_n = 0;
+  long long ai = 0;
+  unsigned long long ar = 0;
+  Sh.di[lane] = 0;
+  Sh.dr[lane] = 0;
+  auto publish = [&]() {
+    if (acc_n > 0) {
+      long long ri = ai + Sh.di[lane];
+      unsigned long long rr = ar + Sh.dr[lane];
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        ai += __shfl_xor_sync(0xffffffffu, ai, o);
+        ar += __shfl_xor_sync(0xffffffffu, ar, o);
+        ri += __shfl_xor_sync(0xffffffffu, ri, o);
+        rr += __shfl_xor_sync(0xffffffffu, rr, o);
+      }
+      if (lane == 0) {
+        FrameState* S = &P.state[acc_f];
+        atomicAdd((unsigned long long*)&S->ll_int[0], (unsigned long long)ai);
+        atomicAdd((unsigned long long*)&S->ll_int[1], (unsigned long long)ri);
+        atomicAdd(&S->ll_frac[0], ar);
+        atomicAdd(&S->ll_frac[1], rr);
+        __threadfence();
+        if (atomicAdd(&S->sv_done, acc_n) == acc_nsv - acc_n) {
+          __threadfence();
+          frame_converge(P, acc_f);
+        }
+      }
+      __syncwarp();
+    }
+    acc_n = 0;
+    ai = 0;
+    ar = 0;
+    Sh.di[lane] = 0;
+    Sh.dr[lane] = 0;
+  };
+  constexpr int kPerItem = G > 0 ? 32 / G : 1;
+  const int knn_items = G > 0 ? (total + kPerItem - 1) / kPerItem : 0;
+  bool knn_more = G > 0;
+  auto knn_step = [&]() {
+    if constexpr (G > 0) {
+      int item = 0;
+      if (lane == 0) item = atomicAdd(&P.work[2], 1);
+      item = __shfl_sync(0xffffffffu, item, 0);
+      if (item < knn_items) {
+        const int gl = lane & (G - 1), gbase = lane - gl;
+        const unsigned gmask = G == 32 ? 0xffffffffu : ((1u << G) - 1u) << gbase;
+        knn_estep_sv<G>(P, item * kPerItem + gbase / G, P.iter + 1, gl, gbase, gmask);
+        __syncwarp();
+      } else {
+        knn_more = false;
+      }
+    }
+  };
+  int s0 = take(0), s1 = take(1), s2 = take(2);
+  fetch_rec(s0, Sh.rec[0]);
+  fetch_rec(s1, Sh.rec[1]);
+  cp_commit();
+  cp_wait_all();
+  __syncwarp();
+  fetch_cand(s0, Sh.rec[0], Sh.cand[0]);
+  cp_commit();
+  // units copied and read by this warp; the unit to copy next and how many of its supervoxel
+  // (the current one, or with on_next the one after) are left to copy; the units copied when
+  // the last records were asked for
+  unsigned gi = 0, gc = 0, g_rec = 0;
+  const float4* src = nullptr;
+  int left = 0, part = 0;
+  bool on_next = false, asked = false;
+  for (int i = 0; s0 >= 0; i++) {
+    // the records asked for a supervoxel ago, which went with the unit copied next
+    if (asked) cp_commit();
+    ls_wait(asked ? 0 : (int)(gi - g_rec));
+    __syncwarp();
+    const LSRec& A = Sh.rec[i % 3];
+    const LSRec& B = Sh.rec[(i + 1) % 3];
+    const LSCand& K = Sh.cand[i & 1];
+    const int nv = A.ll.nv, f = A.ll.frame;
+    const int nu = (nv + kLSUnit - 1) / kLSUnit, gap = nu * kLSUnit - nv;
+    if (!on_next) {  // its copies start here
+      src = P.vox4 + A.ll.v0 + lane - gap;
+      left = nu;
+      part = gap;
+    }
+    on_next = false;
+    const bool run = K.done == 0;
+    if (run && f != acc_f) {  // the sums so far are the previous frame's
+      publish();
+      acc_f = f;
+      acc_nsv = A.ll.frame_nsv;
+    }
+    // the candidates' FP32 constants, a candidate on each of five lanes, and bounds of its n over
+    // the supervoxel's box (each row of R (e - u) lies in an interval there)
+    float b = 0.0f, r00 = 0.0f, least = kInfF, most = kInfF;
+    bool wide = false;
+    float r01 = 0.0f, r02 = 0.0f, r11 = 0.0f, r12 = 0.0f, r22 = 0.0f, k0 = 0.0f, k1 = 0.0f, k2 = 0.0f;
+    if (lane < kJ) {
+      const GaussLL& g = K.g[lane];
+      const double u0 = g.m[0] - (double)A.ll.c0, u1 = g.m[1] - (double)A.ll.c1, u2 = g.m[2] - (double)A.ll.c2;
+      r00 = g.r[0], r01 = g.r[1], r02 = g.r[2], r11 = g.r[3], r12 = g.r[4], r22 = g.r[5];
+      k0 = __double2float_rn((double)r00 * u0 + (double)r01 * u1 + (double)r02 * u2);
+      k1 = __double2float_rn((double)r11 * u1 + (double)r12 * u2);
+      k2 = __double2float_rn((double)r22 * u2);
+      b = __double2float_rn(K.ln_alpha * 1.4426950408889634 - g.b);
+      wide = r02 != 0.0f || r12 != 0.0f;
+      const float h0 = A.ll.h0, h1 = A.ll.h1, h2 = A.ll.h2;
+      const float w0 = fabsf(r00) * h0 + fabsf(r01) * h1 + fabsf(r02) * h2, w1 = fabsf(r11) * h1 + fabsf(r12) * h2,
+                  w2 = fabsf(r22) * h2;
+      const float x0 = fmaxf(fabsf(k0) - w0, 0.0f), x1 = fmaxf(fabsf(k1) - w1, 0.0f), x2 = fmaxf(fabsf(k2) - w2, 0.0f);
+      const float z0 = fabsf(k0) + w0, z1 = fabsf(k1) + w1, z2 = fabsf(k2) + w2;
+      least = x0 * x0 + x1 * x1 + x2 * x2 + b;
+      most = z0 * z0 + z1 * z1 + z2 * z2 + b;
+    }
+    const unsigned fin = __ballot_sync(0xffffffffu, lane < kJ && isfinite(b));
+    const unsigned bad = __ballot_sync(0xffffffffu, lane < kJ && (isnan(b) || b == -kInfF));
+    const unsigned odd = __ballot_sync(0xffffffffu, lane < kJ && isnan(r00) && isfinite(b));
+    const bool w4 = !__any_sync(0xffffffffu, wide);
+    float top = most;  // some candidate's n is at most this everywhere
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) top = fminf(top, __shfl_xor_sync(0xffffffffu, top, o));
+    top = __shfl_sync(0xffffffffu, top, 0);
+    // kept: the candidates that can come within kLSDrop bits of the largest term somewhere
+    const unsigned keep = __ballot_sync(0xffffffffu, lane < kJ && !(least > top + kLSDrop)) & 31u;
+    const int nk = __popc(keep);
+    if (lane < kJ) {  // the kept ones first
+      const unsigned below = (1u << lane) - 1u;
+      int at = (keep >> lane) & 1u ? __popc(keep & below) : nk + __popc(~keep & below);
+      if (nk == 3 && (at == 2 || at == 4)) at = 6 - at;  // the third is the single one
+      float* c = Sh.cst + (at < 4 ? (at >> 1) * 20 + (at & 1) : 40);
+      const int st = at < 4 ? 2 : 1;
+      c[0] = r00;
+      c[st] = r01;
+      c[2 * st] = -k0;
+      c[3 * st] = r11;
+      c[4 * st] = -k1;
+      c[5 * st] = r22;
+      c[6 * st] = -k2;
+      c[7 * st] = b;
+      c[8 * st] = r02;
+      c[9 * st] = r12;
+    }
+    const int form = w4 ? nk : 0;
+    __syncwarp();
+    // what the next supervoxels need
+    fetch_cand(s1, B, Sh.cand[(i + 1) & 1]);
+    if (i > 0) s2 = __shfl_sync(0xffffffffu, s2, 0);  // taken a supervoxel ago
+    fetch_rec(s2, Sh.rec[(i + 2) % 3]);
+    asked = true;
+    const int s3 = s2 >= 0 ? take(i + 3) : -1;
+    if (knn_more) knn_step();
+    // a NaN weight makes the reference's density NaN for every voxel (skipped); no finite weight
+    // means a zero density everywhere
+    const bool compute = run && fin && !bad;
+    const int nnv = s1 >= 0 ? B.ll.nv : 0;
+    unsigned fix = 0;
+    if (compute && !odd) {
+      double lt = 0.0;  // log2 units
+      for (int u = 0; u < nu; u++) {
+        // refill the ring: this supervoxel's units, then the next one's
+        while (gi - gc < kLSRing) {
+          if (left == 0) {
+            if (on_next || nnv == 0) break;
+            on_next = true;
+            left = (nnv + kLSUnit - 1) / kLSUnit;
+            part = left * kLSUnit - nnv;
+            src = P.vox4 + B.ll.v0 + lane - part;
+          }
+          const unsigned dst = ring_a + (gi % kLSRing) * (kLSUnit * 16);
+          if (part == 0) {
+#pragma unroll
+            for (int q = 0; q < kLSUnit / 32; q++) cp_async16_to(dst + 512 * q, src + 32 * q);
+          } else {
+#pragma unroll
+            for (int q = 0; q < kLSUnit / 32; q++) {
+              const bool in = 32 * q + lane >= part;
+              cp_async16_fill(dst + 512 * q, in ? src + 32 * q : P.vox4, in ? 16u : 0u);
+            }
+          }
+          cp_commit();
+          src += kLSUnit;
+          part = 0;
+          left--;
+          gi++;
+          if (asked) {
+            asked = false;
+            g_rec = gi;
+          }
+        }
+        ls_wait((int)(gi - gc) - 1);  // at most the units after this one
+        const float4* slot = &Sh.ring[gc % kLSRing][lane];
+        float s = 0.0f, lmin = kInfF;
+        switch (form) {
+          case 1:
+            ls_unit<1>(Sh.cst, slot, s, lmin);
+            break;
+          case 2:
+            ls_unit<2>(Sh.cst, slot, s, lmin);
+            break;
+          case 3:
+            ls_unit<3>(Sh.cst, slot, s, lmin);
+            break;
+          case 4:
+            ls_unit<4>(Sh.cst, slot, s, lmin);
+            break;
+          case 5:
+            ls_unit<5>(Sh.cst, slot, s, lmin);
+            break;
+          default:
+            ls_unit<0>(Sh.cst, slot, s, lmin);
+            break;
+        }
+        if (__any_sync(0xffffffffu, !(lmin > kLSZero) || isnan(s))) {
+          bool allok = true;
+          s = ls_unit_tested(Sh.cst, slot - lane, u == 0 ? gap : 0, &allok);
+          const bool some = __any_sync(0xffffffffu, !allok);
+          if (some && nu > kLSKept && u >= nu - kLSKept) fix |= 1u << (u - (nu - kLSKept));
+        }
+        gc++;
+        lt += (double)s;
+        if (((nu - 1 - u) & (512 / kLSUnit - 1)) == 0) {  // a block of 512 voxels, from the end
+          lt *= kLn2;
+          const double fl = floor(lt);
+          const long long bi = (long long)fl;
+          const unsigned long long br = (unsigned long long)((lt - fl) * kFracScale);
+          ai += bi;
+          ar += br;
+          if (nu - u > kLSKept) {  // before the kept window
+            Sh.di[lane] -= bi;
+            Sh.dr[lane] -= br;
+          }
+          lt = 0.0;
+        }
+      }
+      if (fix) {
+        long long bi = 0;
+        unsigned long long br = 0;
+        fixed_acc(bi, br, kLn2 * ls_fixup(Sh.cst, P.vox4 + A.ll.v0, nu, kLSUnit - gap, fix));
+        Sh.di[lane] += bi;
+        Sh.dr[lane] += br;
+      }
+    } else {
+      // its units on their way (all that is) are let land and passed over
+      ls_wait(0);
+      gc = gi;
+      if (compute) ls_general(P, A.ll, A.cand, K.ln_alpha, &ai, &ar, &Sh.di[lane], &Sh.dr[lane]);
+    }
+    if (run) acc_n++;
+    s0 = s1, s1 = s2, s2 = s3;
+  }
+  cp_wait_all();
+  publish();
+  while (knn_more) knn_step();
+  if ((G > 0 || total > kLSFixed * W) && lane == 0 && atomicAdd(&P.work[1], 1) == W - 1) {
     P.work[0] = 0;
     P.work[1] = 0;
     P.work[2] = 0;
@@ -2426,7 +2790,7 @@ void launch_order(const DevPlan& P, cudaStream_t st) {
   k_order_scatter<<<div_up(P.max_sv, 256), 256, 0, st>>>(P);
 }
 void launch_moments(const DevPlan& P, cudaStream_t st) {
-  k_ll_pass<false, 0, true><<<P.ll_blocks, kLLWarps * 32, kLLSmemBytes, st>>>(P);
+  k_ll_pass<true><<<P.ll_blocks, kLLWarps * 32, kLLSmemBytes, st>>>(P);
 }
 void launch_knn_estep(const DevPlan& P, cudaStream_t st) {
   const int G = P.knn_group;
@@ -2447,18 +2811,17 @@ void launch_kill_prep(const DevPlan& P, cudaStream_t st) {
   k_kill_prep<<<P.max_gchunks, kGChunk, 0, st>>>(P);
 }
 void launch_ll_pass(const DevPlan& P, int fp64, int knn_group, cudaStream_t st) {
-  const int grid = P.ll_blocks;
   const int bs = kLLWarps * 32;
   if (fp64)
-    k_ll_pass<true, 0, false><<<P.ll_blocks64, bs, kLLSmemBytes, st>>>(P);
+    k_ll_pass<false><<<P.ll_blocks64, bs, kLLSmemBytes, st>>>(P);
   else if (knn_group == 8)
-    k_ll_pass<false, 8, false><<<grid, bs, kLLSmemBytes, st>>>(P);
+    k_ll_stream<8><<<P.ls_blocks, kLSWarps * 32, kLSSmemBytes, st>>>(P);
   else if (knn_group == 16)
-    k_ll_pass<false, 16, false><<<grid, bs, kLLSmemBytes, st>>>(P);
+    k_ll_stream<16><<<P.ls_blocks, kLSWarps * 32, kLSSmemBytes, st>>>(P);
   else if (knn_group == 32)
-    k_ll_pass<false, 32, false><<<grid, bs, kLLSmemBytes, st>>>(P);
+    k_ll_stream<32><<<P.ls_blocks, kLSWarps * 32, kLSSmemBytes, st>>>(P);
   else
-    k_ll_pass<false, 0, false><<<grid, bs, kLLSmemBytes, st>>>(P);
+    k_ll_stream<0><<<P.ls_blocks, kLSWarps * 32, kLSSmemBytes, st>>>(P);
 }
 
 // Host tables reach the device as launch parameters of k_stage (24 KB a launch), so staging
@@ -2494,20 +2857,29 @@ cudaError_t configure_kernels(DevPlan& P, int device) {
   // every form of the voxel pass: its dynamic shared memory, and the blocks per SM its
   // persistent grid is sized for -- the fewest of the FP32 forms and the moment pass, and
   // separately the FP64 form, whose per-warp FP64 constants take more shared memory
-  const void* forms[6] = {(const void*)k_ll_pass<false, 0, false>, (const void*)k_ll_pass<false, 8, false>,
-                          (const void*)k_ll_pass<false, 16, false>, (const void*)k_ll_pass<false, 32, false>,
-                          (const void*)k_ll_pass<false, 0, true>, (const void*)k_ll_pass<true, 0, false>};
+  const void* forms[2] = {(const void*)k_ll_pass<true>, (const void*)k_ll_pass<false>};
   int sms = 0, per = 1 << 30, per64 = 1 << 30;
   cudaError_t e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-  for (int i = 0; i < 6; i++) {
+  for (int i = 0; i < 2; i++) {
     int p = 0;
     if (e == cudaSuccess)
       e = cudaFuncSetAttribute(forms[i], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kLLSmemBytes);
     if (e == cudaSuccess)
       e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&p, forms[i], kLLWarps * 32, kLLSmemBytes);
-    int& m = i < 5 ? per : per64;
+    int& m = i < 1 ? per : per64;
     m = p < m ? p : m;
   }
+  const void* stream_forms[4] = {(const void*)k_ll_stream<0>, (const void*)k_ll_stream<8>,
+                                 (const void*)k_ll_stream<16>, (const void*)k_ll_stream<32>};
+  int pers = 1 << 30;
+  for (const void* fn : stream_forms) {
+    int p = 0;
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kLSSmemBytes);
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&p, fn, kLSWarps * 32, kLSSmemBytes);
+    pers = std::min(pers, p);
+  }
+  // no more blocks than supervoxels: a small plan's warps spread over the SMs
+  P.ls_blocks = std::max(1, std::min(P.max_sv, sms * (pers > 0 && pers < (1 << 30) ? pers : 1)));
   P.ll_blocks = sms * (per > 0 && per < (1 << 30) ? per : 1);
   P.ll_blocks64 = sms * (per64 > 0 && per64 < (1 << 30) ? per64 : 1);
   return e;

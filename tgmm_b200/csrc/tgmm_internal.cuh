@@ -161,11 +161,20 @@ static_assert(sizeof(SvRec) == 128, "SvRec is eight 16-byte chunks");
 // 0 holds r0 voxels, later tiles kVoxTile), its frame and its centroid.
 struct SvLL {
   long long v0;
-  int32_t nv, ntiles, r0, frame, frame_nsv;
+  int32_t nv, ntiles, frame, frame_nsv;
   float c0, c1, c2;
-  int32_t pad[2];
+  float h0, h1, h2;  // the largest |x - c| along each axis (the moment pass)
 };
 static_assert(sizeof(SvLL) == 48, "SvLL is three 16-byte chunks");
+
+// Per-Gaussian record of the FP32 log-likelihood pass, built by the kill step: the upper
+// triangle R (00 01 02 11 12 22) with R'R = nu W log2(e) / 2, log2 of the weight (without the
+// frame's alpha total) and the mean.
+struct GaussLL {
+  float r[6], pad[2];
+  double b, m[3];
+};
+static_assert(sizeof(GaussLL) == 64, "GaussLL is four 16-byte chunks");
 
 struct BatchInfo {
   int32_t n_frames;
@@ -208,12 +217,14 @@ struct DevPlan {
   int32_t* work;   // [0] next supervoxel of the voxel pass, [1] warps that left it
   int32_t ll_blocks;    // resident blocks of the voxel pass's FP32 forms (SMs x blocks per SM)
   int32_t ll_blocks64;  // the same for its FP64 form
+  int32_t ls_blocks;    // blocks of the FP32 log-likelihood pass
   int32_t knn_group;  // lanes per supervoxel of the kNN/E-step (8, 16 or 32)
   int32_t iter;       // the EM iteration a launch belongs to (1-based; set per launch)
   unsigned long long stage_wait_ns;  // wait limit of a voxel tile copy (default 1 s)
   float4* kpos;  // per Gaussian: the float centre the kNN sees (x, y, z; w = 1 live, 0 dead)
   double* ec;   // per Gaussian E-step record, kEcStride doubles: nu W [6], m [3], 3/beta, psi(alpha)+eLD/2
   double* llc;  // per Gaussian, 10 doubles: -nu*W/2 (off-diagonals doubled) [6], log weight [1], m [3]
+  GaussLL* gll; // per Gaussian: the record of the FP32 log-likelihood pass
   // per supervoxel
   int32_t* sv_frame;
   int32_t* sv_order;  // the order in which the voxel passes take supervoxels (k_order_*)
