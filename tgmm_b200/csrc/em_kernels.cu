@@ -1460,7 +1460,7 @@ __device__ __forceinline__ double voxel_ll_fp64(const LLShared64& C, float x0, f
                                                 float c2, bool& ok) {
   const double e0 = (double)x0 - (double)c0, e1 = (double)x1 - (double)c1, e2 = (double)x2 - (double)c2;
   double dens = 0.0;
-#pragma unroll
+#pragma unroll 1
   for (int j = 0; j < kJ; j++) {
     const double d0 = e0 - C.u[j][0], d1 = e1 - C.u[j][1], d2 = e2 - C.u[j][2];
     const double* A = C.A[j];
@@ -1482,6 +1482,7 @@ __device__ __forceinline__ double voxel_ll_fp64(const LLShared64& C, float x0, f
 #ifndef TGMM_LL_WARPS
 #define TGMM_LL_WARPS 8
 #endif
+constexpr int kFp64Parts = 4;                 // parts of a supervoxel in the FP64 log-likelihood
 constexpr int kLLWarps = TGMM_LL_WARPS;       // warps per block of the voxel pass
 constexpr int kLLTile = kVoxTile;             // voxels per tile (kVoxTile / 32 per lane)
 constexpr int kLLStages = TGMM_LL_STAGES;     // tile slots per warp
@@ -1646,32 +1647,30 @@ struct VoxelEval64 {
   __device__ __forceinline__ static bool ok(double l) { return l > -kInf; }
 };
 
-// One staged tile: lane voxels o = u*32 + lane, sht[c] the offset of component c in the
-// slot.  kFull: all kLLTile voxels present (else the first rem).  allok turns false when
-// a present voxel has a zero density.
-template <bool kFull>
+// One staged tile: lane voxels o = u*32 + lane < rem, sht[c] the offset of component c in the
+// slot.  allok turns false when a present voxel has a zero density.
+// Rolled (as are the candidates in voxel_ll_fp64): unrolled by eight and five the kernel missed
+// the instruction cache six times as often as it issued.
 __device__ __forceinline__ void ll_tile(const VoxelEval64& eval, const float* __restrict__ slot, const int* sht, int rem,
                                         float c0, float c1, float c2, double& tsum, bool& allok) {
   const int lane = threadIdx.x & 31;
-  const float* bx = slot + sht[0] + lane;
-  const float* by = slot + kLLSpan + sht[1] + lane;
-  const float* bz = slot + 2 * kLLSpan + sht[2] + lane;
-  const float* bi = slot + 3 * kLLSpan + sht[3] + lane;
-#pragma unroll
-  for (int u = 0; u < kLLTile / 32; u++) {
-    if (!kFull && u * 32 >= rem) break;
-    const double l = eval(bx[32 * u], by[32 * u], bz[32 * u], c0, c1, c2);
+  const float* bx = slot + sht[0];
+  const float* by = slot + kLLSpan + sht[1];
+  const float* bz = slot + 2 * kLLSpan + sht[2];
+  const float* bi = slot + 3 * kLLSpan + sht[3];
+#pragma unroll 2
+  for (int o = lane; o < rem; o += 32) {
+    const double l = eval(bx[o], by[o], bz[o], c0, c1, c2);
     const bool ok = VoxelEval64::ok(l);
-    const bool in = kFull || u * 32 + lane < rem;
-    allok = allok && (ok || !in);
-    tsum += (in && ok) ? (double)bi[32 * u] * l : 0.0;
+    allok = allok && ok;
+    tsum += ok ? (double)bi[o] * l : 0.0;
   }
 }
 
 // A kept voxel (one of the last 1024 of a supervoxel above 1024 voxels) with a zero
 // density: the reference thread of its stride still holds the last voxel of the stride
 // with a positive density (GMEMupdateCUDA.cu:1961-1962).  Rare; reads global memory.
-__device__ __forceinline__ double ll_walk_back(const VoxelEval64& eval, const SvRec& R, int i, float c0, float c1, float c2) {
+__device__ __noinline__ double ll_walk_back(const VoxelEval64& eval, const SvRec& R, int i, float c0, float c1, float c2) {
   const float* v[4];
 #pragma unroll
   for (int c = 0; c < 4; c++) v[c] = reinterpret_cast<const float*>(R.lo0[c]) + ((R.nf[c] >> 16) & 3);
@@ -1685,7 +1684,7 @@ __device__ __forceinline__ double ll_walk_back(const VoxelEval64& eval, const Sv
 // The kept tiles (bit t - (nt - kKeptTiles) of `mask`) that hold voxels of zero density, after the
 // supervoxel's tiles: their voxels are read again from global memory and each one of zero
 // density adds the walk-back value.  Rare.
-__device__ __forceinline__ double ll_fixup(const VoxelEval64& eval, const SvRec& R, unsigned mask, float c0, float c1,
+__device__ __noinline__ double ll_fixup(const VoxelEval64& eval, const SvRec& R, unsigned mask, float c0, float c1,
                                            float c2) {
   const int lane = threadIdx.x & 31;
   const float* v[4];
@@ -1777,10 +1776,7 @@ __device__ __forceinline__ void ll_consume(const VoxelEval64& eval, const float*
   const int rem = t == 0 ? r0 : kLLTile;
   double tsum = 0.0;
   bool allok = true;
-  if (rem == kLLTile)
-    ll_tile<true>(eval, slot, sht, rem, c0, c1, c2, tsum, allok);
-  else
-    ll_tile<false>(eval, slot, sht, rem, c0, c1, c2, tsum, allok);
+  ll_tile(eval, slot, sht, rem, c0, c1, c2, tsum, allok);
   lt += tsum;
   if (t >= nt - kKeptTiles) {
     lr += tsum;
@@ -1840,7 +1836,11 @@ __device__ void frame_converge(const DevPlan& P, int f) {
 template <bool kMom>
 __global__ void __launch_bounds__(kLLWarps * 32, kLLBlocks) k_ll_pass(DevPlan P) {
   constexpr bool kRec = true, kLLr = kMom, kCand = !kMom, kFp64 = !kMom;
-  const int total = P.info->total_sv;
+  // the FP64 log-likelihood takes a supervoxel in kParts parts (part p: tiles p, p + kParts, ...):
+  // at one warp a supervoxel its time was that of the largest one (2000 supervoxels, 1.4 M voxels:
+  // 106 us in one part, 81 in two, 72 in four, 73 in eight; 174 before it was rolled, see ll_tile)
+  constexpr int kParts = kMom ? 1 : kFp64Parts;
+  const int total = P.info->total_sv * kParts;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   __shared__ LLShared64 sh64[kFp64 ? kLLWarps : 1];
   extern __shared__ __align__(128) unsigned char ll_smem[];
@@ -1882,10 +1882,11 @@ __global__ void __launch_bounds__(kLLWarps * 32, kLLBlocks) k_ll_pass(DevPlan P)
   FrameState* S = nullptr;
   bool failed = false;
   // tickets: the current, the next, and (lane 0) the one after
-  // a ticket t is the supervoxel sv_order[t] (each frame's largest first), total at the end
+  // a ticket t is part t % kParts of the supervoxel sv_order[t / kParts] (each frame's largest
+  // first), as supervoxel * kParts + part, total at the end
   auto take = [&]() {
     const int t = atomicAdd(&P.work[0], 1);
-    return t < total ? P.sv_order[t] : total;
+    return t < total ? P.sv_order[t / kParts] * kParts + t % kParts : total;
   };
   int tk = 0;
   if (lane == 0) tk = take();
@@ -1895,8 +1896,8 @@ __global__ void __launch_bounds__(kLLWarps * 32, kLLBlocks) k_ll_pass(DevPlan P)
   if (lane == 0 && sn < total) tk = take();
   auto frame_of = [](const LLRec& A) { return A.rec.frame; };
   if (sc < total) {
-    ll_fetch_a<kRec, kLLr, kCand>(P, RA[0], sc);
-    if (sn < total) ll_fetch_a<kRec, kLLr, kCand>(P, RA[1], sn);
+    ll_fetch_a<kRec, kLLr, kCand>(P, RA[0], sc / kParts);
+    if (sn < total) ll_fetch_a<kRec, kLLr, kCand>(P, RA[1], sn / kParts);
     cp_commit();
     cp_wait_all();
     __syncwarp();
@@ -1913,12 +1914,14 @@ __global__ void __launch_bounds__(kLLWarps * 32, kLLBlocks) k_ll_pass(DevPlan P)
     const int s2 = __shfl_sync(0xffffffffu, tk, 0);
     if (lane == 0 && s2 < total) tk = take();
     if (!kMom && sn < total) ll_fetch_b(P, NA, frame_of(NA), RB[(i + 1) & 1]);
-    if (s2 < total) ll_fetch_a<kRec, kLLr, kCand>(P, RA[(i + 2) % 3], s2);
+    if (s2 < total) ll_fetch_a<kRec, kLLr, kCand>(P, RA[(i + 2) % 3], s2 / kParts);
     cp_commit();
     int in = 0;
-    const int n_nt = sn < total ? NA.rec.ntiles : 0;  // the next one's tiles may start early
+    // this part's tiles, and the next one's, which may start early
+    const int part = sc % kParts, part_n = sn % kParts;
+    const int n_nt = sn < total ? (NA.rec.ntiles - part_n + kParts - 1) / kParts : 0;
     const int nv = CA.rec.nv, nt = CA.rec.ntiles;
-    const int f = frame_of(CA), nsv = CA.rec.frame_nsv;
+    const int f = frame_of(CA), nsv = CA.rec.frame_nsv * kParts;
     const float c0 = CA.rec.c0, c1 = CA.rec.c1, c2 = CA.rec.c2;
     S = &P.state[f];
     int pk[4] = {0, 0, 0, 0};  // SoA slot offsets of the components: tile 0 in bits 0-1, later tiles in bits 4-5
@@ -1934,7 +1937,7 @@ __global__ void __launch_bounds__(kLLWarps * 32, kLLBlocks) k_ll_pass(DevPlan P)
       while (gi < gc + kLLStages) {
         const bool mine = ic < ntr;
         if (!mine && in >= n_nt) break;
-        const int tt = mine ? ic++ : in++;
+        const int tt = mine ? part + kParts * ic++ : part_n + kParts * in++;
         if (lane == 0) {
           const unsigned q = gi % kLLStages;
           ll_issue(mine ? CA.rec : NA.rec, tt, wbuf + q * kLLSlotFloats, bar0 + 8 * q);
@@ -2000,7 +2003,7 @@ __global__ void __launch_bounds__(kLLWarps * 32, kLLBlocks) k_ll_pass(DevPlan P)
     double lt = 0.0, lr = 0.0;
     unsigned fix = 0;  // kept tiles with voxels of zero density
     // a finished frame issues no more tiles; those issued early are consumed unread
-    const int ntr = run ? nt : ic;
+    const int ntr = run ? (nt - part + kParts - 1) / kParts : ic;
     // the supervoxel's tiles and, rarely, the kept window's zero-density voxels
     const VoxelEval64 eval{Q};
     for (int t = 0; t < ntr; t++) {
@@ -2009,7 +2012,7 @@ __global__ void __launch_bounds__(kLLWarps * 32, kLLBlocks) k_ll_pass(DevPlan P)
         failed = true;
         break;
       }
-      if (compute) ll_consume(eval, slot, pk, t, nt, nv, r0, c0, c1, c2, lt, lr, fix);
+      if (compute) ll_consume(eval, slot, pk, part + kParts * t, nt, nv, r0, c0, c1, c2, lt, lr, fix);
       gc++;
     }
     if (!failed && fix) lr += ll_fixup(eval, CA.rec, fix, c0, c1, c2);
