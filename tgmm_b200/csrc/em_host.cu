@@ -368,6 +368,8 @@ int stage_batch(TgmmPlan* P, int32_t n, const TgmmFrame* fr, TgmmGaussian* const
       D.scale[d] = prm->scale[d];
       D.reg_scale[d] = reg_zero ? prm->scale[d] : prm->reg_scale[d];
     }
+    for (int i = 0, e = 0; i < 3; i++)
+      for (int j = i; j < 3; j++) D.reg_inv_s2[e++] = 1.0 / (double)(D.reg_scale[i] * D.reg_scale[j]);
     D.w4dof = prm->w4dof ? 1 : 0;
     D.lambda_min = prm->lambda_min;
     D.lambda_max = prm->lambda_max;

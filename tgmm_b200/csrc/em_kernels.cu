@@ -370,7 +370,8 @@ __device__ __forceinline__ int ref_cell_of(const FrameState& S, const FrameDesc&
 __device__ __forceinline__ double write_records(const DevPlan& P, const FrameDesc& D, int k, int parity, bool dead,
                                                 const double* W, double nu, double alpha, double beta,
                                                 const double* m, bool track, float4 o = float4{}) {
-  const double psa = digamma(alpha);
+  double corr;
+  const double psa = alpha > 1e-6 ? log(digamma_shift(alpha, &corr)) - corr : digamma(alpha);
   const double eld = dead ? -1e32 : expected_log_det(W, nu);
   gcomp(P, G_PSIA0 + parity, k) = psa;
   gcomp(P, G_ELD0 + parity, k) = eld;
@@ -389,7 +390,7 @@ __device__ __forceinline__ double write_records(const DevPlan& P, const FrameDes
   L[3] = -0.5 * nu * W[3];
   L[4] = -nu * W[4];
   L[5] = -0.5 * nu * W[5];
-  L[6] = 0.5 * log(det3(W) * nu * nu * nu) - 1.5 * kLnTwoPi + log(alpha);
+  L[6] = 0.5 * log(det3(W) * nu * nu * nu * (alpha * alpha)) - 1.5 * kLnTwoPi;
   L[7] = m[0];
   L[8] = m[1];
   L[9] = m[2];
@@ -1223,6 +1224,7 @@ __global__ void __launch_bounds__(kMChunk) k_mstep_update(DevPlan P) {
       rc.lambda_min = D.lambda_min;
       rc.lambda_max = D.lambda_max;
       rc.max_exc = D.max_exc;
+      rc.inv_s2 = D.reg_inv_s2;
       regularize_W(W, nu, rc);
       for (int e = 0; e < 6; e++) gcomp(P, G_W0 + e, k) = W[e];
       for (int e = 0; e < 6; e++) nanw = nanw || isnan(W[e]);

@@ -92,6 +92,7 @@ struct FrameDesc {
   float scale[3];      // kNN distance scale
   float reg_scale[3];  // regularisation scale
   int32_t w4dof;
+  double reg_inv_s2[6];  // 1 / (s_i s_j) of the regularisation scale (entries 00 01 02 11 12 22)
   double lambda_min, lambda_max, max_exc, tol;
   int32_t max_iter, ll_mode, ll_prec, frame_id;
 };

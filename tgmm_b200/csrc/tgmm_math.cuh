@@ -13,9 +13,12 @@
 #define TG_HD static inline
 #endif
 
-// Device code scales by one reciprocal per shared denominator instead of dividing each
-// term (about 1 ulp apart, shorter FP64 chains); host code keeps the plain divisions with
-// which the synthetic generator's seeded workloads were pinned.
+// Device code scales by one reciprocal (or reciprocal square root) per shared denominator
+// instead of dividing each term, compares ratios as products, and takes one logarithm of a
+// product instead of several (each about 1 ulp apart): a Gaussian's update is one thread's
+// chain of FP64 operations, some 20 instructions a division and 45 a logarithm, and the whole
+// grid is less than one wave.  Host code keeps the plain forms with which the synthetic
+// generator's seeded workloads were pinned.
 #if defined(__CUDA_ARCH__)
 #define TG_RCP 1
 #else
@@ -49,6 +52,21 @@ TG_HD double digamma_pos(double x) {
   double acc = log(x) - 0.5 * inv - num / den;
   acc -= t * (1.0 / 12 - t * (1.0 / 120 - t * (1.0 / 252 - t * (1.0 / 240 - t * (1.0 / 132)))));
   return acc;
+}
+
+// psi(x) = log(X) - corr for 1e-6 < x: the argument X after the recurrence and the rest of the
+// series, with one division for 1/X and the recurrence's fraction.
+TG_HD double digamma_shift(double x, double* corr) {
+  double num = 0.0, den = 1.0;
+  while (x < 12.0) {
+    num = num * x + den;
+    den *= x;
+    x += 1.0;
+  }
+  const double r = 1.0 / (x * den), inv = den * r, t = inv * inv;
+  *corr = r * (0.5 * den + num * x) +
+          t * (1.0 / 12 - t * (1.0 / 120 - t * (1.0 / 252 - t * (1.0 / 240 - t * (1.0 / 132)))));
+  return x;
 }
 
 // psi over the reals: -1e300 at the poles, reflection for negative arguments.
@@ -87,21 +105,24 @@ TG_HD void inv3(const double* w, double* o) {
 }
 
 TG_HD bool unit3(double* a) {
+#if TG_RCP
+  const double n2 = a[0] * a[0] + a[1] * a[1] + a[2] * a[2];
+  if (!(n2 > 1e-24)) return false;
+  const double r = rsqrt(n2);
+  a[0] *= r;
+  a[1] *= r;
+  a[2] *= r;
+  return true;
+#else
   const double n = sqrt(a[0] * a[0] + a[1] * a[1] + a[2] * a[2]);
   if (n > 1e-12) {
-    if (TG_RCP) {
-      const double r = 1.0 / n;
-      a[0] *= r;
-      a[1] *= r;
-      a[2] *= r;
-    } else {
-      a[0] /= n;
-      a[1] /= n;
-      a[2] /= n;
-    }
+    a[0] /= n;
+    a[1] /= n;
+    a[2] /= n;
     return true;
   }
   return false;
+#endif
 }
 
 // Closed-form eigen-decomposition of a symmetric 3x3 matrix: eigenvalues from the
@@ -126,15 +147,19 @@ TG_HD void eig3(const double* w, double* d, double* v) {
     const double q = 0.5 * (a0 * (a3 * a5 - w[4] * w[4]) - w[1] * (w[1] * a5 - w[2] * w[4]) +
                             w[2] * (w[1] * w[4] - w[2] * a3));
     const double p = (2.0 * (w[1] * w[1] + w[2] * w[2] + w[4] * w[4]) + a0 * a0 + a3 * a3 + a5 * a5) / 6.0;
+#if TG_RCP
+    const double ir = rsqrt(p), r = p * ir, ratio = q * (ir * ir * ir);
+#else
     const double r = sqrt(p);
-    const double ratio = TG_RCP ? q / (p * r) : q / pow(p, 1.5);
+    const double ratio = q / pow(p, 1.5);
+#endif
     double phi;
     if (ratio <= -1)
       phi = 3.14159265358979311600 / 3.0;
     else if (ratio >= 1)
       phi = 0;
     else
-      phi = acos(ratio) / 3.0;
+      phi = TG_RCP ? acos(ratio) * (1.0 / 3.0) : acos(ratio) / 3.0;
     double s, c;
     if (TG_RCP) {
       sincos(phi, &s, &c);
@@ -231,6 +256,7 @@ struct RegConst {
   float scale[3];
   int w4dof;
   double lambda_min, lambda_max, max_exc;
+  const double* inv_s2;  // device code: 1 / (s_i s_j) of the six entries
 };
 
 // Precision-matrix regularisation (GMEMregularizeWkKernel, GMEMupdateCUDA.cu:1693-1809):
@@ -245,8 +271,11 @@ TG_HD void regularize_W(double* Wk, double nu, const RegConst& rc) {
   const double lo = TG_RCP ? rc.lambda_min * inu : rc.lambda_min / nu;
   double W[6];
   for (int e = 0; e < 6; e++) {
-    const double s2 = (double)(rc.scale[ia[e]] * rc.scale[ib[e]]);
-    W[e] = TG_RCP ? Wk[e] * (1.0 / s2) : Wk[e] / s2;
+#if TG_RCP
+    W[e] = Wk[e] * rc.inv_s2[e];
+#else
+    W[e] = Wk[e] / (double)(rc.scale[ia[e]] * rc.scale[ib[e]]);
+#endif
   }
   if (rc.w4dof) {
     W[2] = 0.0;
@@ -258,11 +287,19 @@ TG_HD void regularize_W(double* Wk, double nu, const RegConst& rc) {
   for (int i = 0; i < 3; i++) d[i] = d[i] < lo ? lo : d[i];
   const int pa[3] = {0, 0, 1}, pb[3] = {1, 2, 2};
   for (int q = 0; q < 3; q++) {
+#if TG_RCP
+    // the clamp above left them positive
+    if (d[pa[q]] > rc.max_exc * d[pb[q]])
+      d[pa[q]] = rc.max_exc * d[pb[q]];
+    else if (d[pb[q]] > rc.max_exc * d[pa[q]])
+      d[pb[q]] = rc.max_exc * d[pa[q]];
+#else
     const double r = d[pa[q]] / d[pb[q]];
     if (r > rc.max_exc)
       d[pa[q]] = rc.max_exc * d[pb[q]];
     else if (1. / r > rc.max_exc)
       d[pb[q]] = rc.max_exc * d[pa[q]];
+#endif
   }
   W[0] = d[0] * v[0] * v[0] + d[1] * v[3] * v[3] + d[2] * v[6] * v[6];
   W[3] = d[0] * v[1] * v[1] + d[1] * v[4] * v[4] + d[2] * v[7] * v[7];
@@ -278,6 +315,13 @@ TG_HD void regularize_W(double* Wk, double nu, const RegConst& rc) {
 // E[ln |Lambda|] = 3 ln 2 + ln det W + sum_{i=0..2} psi((nu + 1 - i)/2)
 // (GMEMupdateCUDA.cu:553-576; the index starts at 0 as in the reference).
 TG_HD double expected_log_det(const double* W, double nu) {
+#if TG_RCP
+  if (nu > 1.0 + 2e-6) {
+    double c[3], x = det3(W);
+    for (int i = 0; i < 3; i++) x *= digamma_shift(0.5 * (nu + 1.0 - i), &c[i]);
+    return 3.0 * kLn2 + log(x) - ((c[0] + c[1]) + c[2]);
+  }
+#endif
   double out = 3.0 * kLn2 + log(det3(W));
   for (int i = 0; i < 3; i++) out += digamma(0.5 * (nu + 1.0 - i));
   return out;
