@@ -1061,8 +1061,6 @@ __global__ void __launch_bounds__(kMChunk) k_mstep_update(DevPlan P) {
   const int c = blockIdx.x >> 1, half = blockIdx.x & 1;
   if (c >= P.info->n_gchunks) return;
   const GChunk ch = P.gchunks[c];
-  if (P.state[ch.frame].done) return;
-  const FrameDesc D = load_desc(P, ch.frame);
   __shared__ int s_ovf[kMChunk];
   __shared__ int s_novf;
   __shared__ double s_ovf_acc[kMChunk][10];
@@ -1071,14 +1069,6 @@ __global__ void __launch_bounds__(kMChunk) k_mstep_update(DevPlan P) {
   __shared__ double shd[kMChunk / 32];
   __shared__ int s_bk[kBucketCap][kMChunk];  // each thread's bucket, one column per thread
   if (threadIdx.x == 0) s_novf = 0;
-  __syncthreads();
-  {
-    // the grid of this frame was read by this iteration's kNN and is refilled by the kill
-    // step: its 2*n_gchunks M-step blocks clear it
-    const int nb = 2 * D.n_gchunks, rank = 2 * (c - D.gchunk_base) + half;
-    const int ncell = P.state[ch.frame].n_cells;
-    for (int i = rank * kMChunk + threadIdx.x; i < ncell; i += nb * kMChunk) P.cell_cnt[D.cell_base + i] = 0;
-  }
   const int k = ch.g_begin + half * kMChunk + threadIdx.x;
   const bool valid = k < ch.g_end;
   double A[10];
@@ -1086,14 +1076,21 @@ __global__ void __launch_bounds__(kMChunk) k_mstep_update(DevPlan P) {
   for (int i = 0; i < 10; i++) A[i] = 0.0;
   double mref[3] = {0, 0, 0};
   bool ovf = false;
-  // the Gaussian's own inputs of the update, loaded ahead of the bucket work so that they
-  // arrive beside it: the prior (m_o also re-centres the pairs), its fixed flag, this
-  // iteration's E[ln|Lambda|] (the kill step's NaN test) and the centre the kNN saw
+  // the Gaussian's own inputs of the update, loaded ahead of the frame's state and of the bucket
+  // work so that they arrive beside them: the prior (m_o also re-centres the pairs), its fixed
+  // flag, this iteration's E[ln|Lambda|] (the kill step's NaN test), the centre the kNN saw, and
+  // the bucket's count and first eight entries (entries past the count are stale and unused; the
+  // bucket rows are 128-byte aligned)
   const int cur = P.iter & 1, nxt = cur ^ 1;
   double bo = 0.0, nuo = 0.0, alo = 0.0, Wo[6] = {0, 0, 0, 0, 0, 0}, eld_cur = 0.0, alpha_old = 0.0;
   bool fixed_k = false;
   float4 kp_old = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  int4 b0 = make_int4(0, 0, 0, 0), b1 = b0;
+  int n = 0;
+  const int* bk = P.bucket + (int64_t)(valid ? k : 0) * kBucketCap;
   if (valid) {
+    n = P.bcnt[k];
+    b0 = *reinterpret_cast<const int4*>(bk), b1 = *reinterpret_cast<const int4*>(bk + 4);
     for (int d = 0; d < 3; d++) mref[d] = gcomp(P, G_MO0 + d, k);
     bo = gcomp(P, G_BETAO, k);
     nuo = gcomp(P, G_NUO, k);
@@ -1103,11 +1100,18 @@ __global__ void __launch_bounds__(kMChunk) k_mstep_update(DevPlan P) {
     alpha_old = gcomp(P, G_ALPHA, k);
     fixed_k = P.fixed[k] != 0;
     kp_old = P.kpos[k];
-    // the bucket's first eight entries load beside its count (entries past the count are
-    // stale and unused; the bucket rows are 128-byte aligned)
-    const int* bk = P.bucket + (int64_t)k * kBucketCap;
-    const int4 b0 = *reinterpret_cast<const int4*>(bk), b1 = *reinterpret_cast<const int4*>(bk + 4);
-    const int n = P.bcnt[k];
+  }
+  const FrameDesc D = load_desc(P, ch.frame);
+  const int ncell = P.state[ch.frame].n_cells;
+  if (P.state[ch.frame].done) return;
+  __syncthreads();
+  {
+    // the grid of this frame was read by this iteration's kNN and is refilled by the kill
+    // step: its 2*n_gchunks M-step blocks clear it
+    const int nb = 2 * D.n_gchunks, rank = 2 * (c - D.gchunk_base) + half;
+    for (int i = rank * kMChunk + threadIdx.x; i < ncell; i += nb * kMChunk) P.cell_cnt[D.cell_base + i] = 0;
+  }
+  if (valid) {
     P.bcnt[k] = 0;
     const int t = threadIdx.x;
     if (n > kBucketCap) {
