@@ -594,7 +594,7 @@ __global__ void __launch_bounds__(256) k_order_scatter(DevPlan P) {
 // ===========================================================================
 constexpr int kKnnWarps = 4;  // warps per block; the lanes per supervoxel (G) come from the plan
 #ifndef TGMM_KNN_BLOCKS
-#define TGMM_KNN_BLOCKS 5  // 96 registers: the list path fits more warps; the rare grid search spills a little
+#define TGMM_KNN_BLOCKS 8  // 64 registers: the list path of 20,000 supervoxels in one wave at 4 or 8 lanes
 #endif
 constexpr int kKnnBlocks = TGMM_KNN_BLOCKS;  // resident blocks per SM the kNN/E-step is compiled for
 
@@ -646,6 +646,131 @@ __device__ __forceinline__ void group_max_pair(float& d, int& i, unsigned gmask)
       i = oi;
     }
   }
+}
+
+// Where a query sits in the grid: its cell, the gaps to that cell's faces, and the float
+// rounding of the scaled coordinates and faces (eps0; distances of d add 1e-6 d).
+struct GridPlace {
+  int c[3];
+  float f0[3], f1[3];  // gaps to the cell's lower and upper faces
+  float delta, eps0;   // the smallest gap; the rounding
+  __device__ __forceinline__ GridPlace(float q0, float q1, float q2, const float* s, const GridGeom& g) {
+    const float y[3] = {q0 * s[0], q1 * s[1], q2 * s[2]};
+    float ymax = 0.0f;
+    delta = kInfF;
+#pragma unroll
+    for (int a = 0; a < 3; a++) {
+      c[a] = cell_coord(y[a], g.lo[a], g.inv_h, g.dims[a]);
+      f0[a] = y[a] - (g.lo[a] + c[a] * g.h);
+      f1[a] = (g.lo[a] + (c[a] + 1) * g.h) - y[a];
+      delta = fminf(delta, fminf(f0[a], f1[a]));
+      ymax = fmaxf(ymax, fabsf(y[a]));
+    }
+    delta = fmaxf(delta, 0.0f);
+    eps0 = 4e-3f + 1e-6f * ymax;
+  }
+  // A squared distance below which every reference lies in the cells at Chebyshev distance
+  // <= r (0: none is known).  References outside the box sit in the boundary cells, farther
+  // from a query inside it than those cells.
+  __device__ __forceinline__ float bound2(int r, float h) const {
+    const float lb = r * h + delta, m = lb - (eps0 + 1e-6f * lb);
+    return m > 0.0f ? m * m : 0.0f;
+  }
+  // squared lower bound of the distance along axis a to the cells at offset o
+  __device__ __forceinline__ float gap2(int a, int o, float h) const {
+    const float gap = o < 0 ? f0[a] + (float)(-o - 1) * h : f1[a] + (float)(o - 1) * h;
+    const float m = fmaxf(gap - eps0 - 1e-6f * gap, 0.0f);
+    return o == 0 ? 0.0f : m * m;
+  }
+};
+
+// Up to N nearest, at least kJ, by collecting instead of keeping sorted lists: the group's lanes
+// put every reference within a limit into `keep` (shared memory, unsorted), then each ranks its
+// share against all.  The limit is a distance that should hold 2 N at the grid's mean density
+// and for which the 27 cells around the query are complete, on fewer than kJ a wider one; or
+// (td0, ti0), a (distance, index) no smaller than the N-th neighbour's, where that is nearer.
+// Every reference not returned is at the squared
+// distance `rest` or farther.  False when the cells within two of the query's do not settle it:
+// the caller runs the ring search.  20,000 supervoxels that all search: 72 us a launch with
+// sorted lists of eight per lane and their merges, 49 us this way (8 lanes).
+constexpr int kKnnKeep = 64;  // references kept; N more places hold the result
+template <int G, int N>
+__device__ __forceinline__ bool knn_group_collect(float q0, float q1, float q2, const float* s, const GridGeom& g,
+                                                  const int32_t* __restrict__ ccnt, const float4* __restrict__ refs,
+                                                  float2* keep, int* count, TopN<N>& best, float& rest,
+                                                  unsigned gmask, int gl, float td0, int ti0) {
+  const GridPlace p(q0, q1, q2, s, g);
+  const float near2 = p.bound2(1, g.h), far2 = p.bound2(2, g.h);
+  float lim = fminf(1.17f * g.h * g.h, near2);  // (16 3 / (4 pi 3))^(2/3) h^2
+  const bool known = td0 < lim;
+  if (known) lim = td0;
+  auto scan = [&](int cell, int e) {
+    const float4* cr = refs + (int64_t)cell * kCellCap;
+    for (int k = 0; k < e; k++) {
+      const float4 rr = cr[k];
+      const float d = knn_dist(q0, q1, q2, rr.x, rr.y, rr.z, s);
+      if (known ? !before(td0, ti0, d, __float_as_int(rr.w)) : d < lim) {
+        const int at = atomicAdd(count, 1);
+        if (at < kKnnKeep) keep[at] = make_float2(d, rr.w);
+      }
+    }
+  };
+  // the cell at an offset, or -1 outside the grid or past the limit
+  auto cell_at = [&](int dx, int dy, int dz) {
+    const int x = p.c[0] + dx, yy = p.c[1] + dy, z = p.c[2] + dz;
+    const bool in = x >= 0 && yy >= 0 && z >= 0 && x < g.dims[0] && yy < g.dims[1] && z < g.dims[2] &&
+                    !(p.gap2(0, dx, g.h) + p.gap2(1, dy, g.h) + p.gap2(2, dz, g.h) > lim);
+    return in ? (z * g.dims[1] + yy) * g.dims[0] + x : -1;
+  };
+  for (int tries = 0; tries < 3; tries++) {
+    const bool one = lim <= near2;
+    if (gl == 0) *count = 0;
+    __syncwarp(gmask);
+    if (one) {
+      constexpr int kPer = (27 + G - 1) / G;
+      int cq[kPer], eq[kPer];
+#pragma unroll
+      for (int q = 0; q < kPer; q++) {
+        const int idx = gl + G * q;
+        cq[q] = idx < 27 ? cell_at(idx % 3 - 1, (idx / 3) % 3 - 1, idx / 9 - 1) : -1;
+        eq[q] = cq[q] >= 0 ? min(ccnt[cq[q]], kCellCap) : 0;
+      }
+#pragma unroll
+      for (int q = 0; q < kPer; q++) scan(cq[q], eq[q]);
+    } else {
+      for (int idx = gl; idx < 125; idx += G) {
+        const int c = cell_at(idx % 5 - 2, (idx / 5) % 5 - 2, idx / 25 - 2);
+        if (c >= 0) scan(c, min(ccnt[c], kCellCap));
+      }
+    }
+    __syncwarp(gmask);
+    const int n = *count;
+    if (n > kKnnKeep) return false;
+    if (n >= kJ) {
+      for (int a = gl; a < n; a += G) {
+        const float2 e = keep[a];
+        int rank = 0;
+        for (int o = 0; o < n; o++) {
+          const float2 f = keep[o];
+          rank += before(f.x, __float_as_int(f.y), e.x, __float_as_int(e.y)) ? 1 : 0;
+        }
+        if (rank < N) keep[kKnnKeep + rank] = e;
+      }
+      __syncwarp(gmask);
+#pragma unroll
+      for (int j = 0; j < N; j++) {
+        const float2 e = j < n ? keep[kKnnKeep + j] : make_float2(kInfF, __int_as_float(0x7fffffff));
+        best.d[j] = e.x;
+        best.i[j] = __float_as_int(e.y);
+      }
+      rest = n < N ? lim : best.d[N - 1];
+      return true;
+    }
+    __syncwarp(gmask);  // every lane has read the count
+    if (known || !(lim < far2)) return false;
+    lim = fminf(lim * (n == 0 ? 4.0f : 2.0f), far2);
+  }
+  return false;
 }
 
 // Exact N nearest over the grid rings.  (td0, ti0): a (distance, index) no smaller than
@@ -747,10 +872,12 @@ __device__ void knn_group_search(float q0, float q1, float q2, const float* s, c
 // of the group whose first lane is gbase).  Its candidates and responsibilities go to the
 // buffers of the iteration's parity.  It reads the frame state the kill step of iteration
 // it - 1 left (grid, neighbour-list bound, psi of the alpha total) and the done flag:
-// when it runs inside the voxel pass of iteration it - 1 (k_ll_pass), that pass may end
+// when it runs inside the voxel pass of iteration it - 1 (k_ll_stream), that pass may end
 // the frame meanwhile, and the results of an iteration that does not run are never read.
+// keep, count: the shared scratch of the group for a search (nullptr: the ring search).
 template <int G>
-__device__ __forceinline__ void knn_estep_sv(const DevPlan& P, int s, int it, int gl, int gbase, unsigned gmask) {
+__device__ __forceinline__ void knn_estep_sv(const DevPlan& P, int s, int it, int gl, int gbase, unsigned gmask,
+                                             float2* keep, int* count) {
   static_assert(G >= 4 && G <= 32 && (G & (G - 1)) == 0, "groups of 4 to 32 lanes");
   // per lane: list members gl + G q (q < kM) and candidates gl + G q (q < kC); one of each
   // for groups of 8 or more lanes
@@ -849,7 +976,10 @@ __device__ __forceinline__ void knn_estep_sv(const DevPlan& P, int s, int it, in
     }
     TopN<kNbr> nb;
     topn_init<kNbr>(nb);
-    if (grid_ok)
+    float rest = -1.0f;  // squared distance of what the list leaves out, where it is not its last's
+    if (grid_ok && !(keep && knn_group_collect<G, kNbr>(q0, q1, q2, D.scale, g, P.cell_cnt + D.cell_base,
+                                                        P.cell_refs + (int64_t)D.cell_base * kCellCap, keep, count, nb,
+                                                        rest, gmask, gl, td0, ti0)))
       knn_group_search<G, kNbr>(q0, q1, q2, D.scale, g, P.cell_cnt + D.cell_base,
                                 P.cell_refs + (int64_t)D.cell_base * kCellCap, nb, gmask, gl, td0, ti0);
     if (!grid_ok || !(nb.d[kJ - 1] < kInfF)) {
@@ -879,8 +1009,8 @@ __device__ __forceinline__ void knn_estep_sv(const DevPlan& P, int s, int it, in
         if (gl + G * m == q) mi = nb.i[q];
       if (gl + G * m < kNbr) P.nbr[(int64_t)s * kNbr + gl + G * m] = mi == 0x7fffffff ? mi : D.g_base + mi;
     }
-    if (gl == 0)
-      P.nbr_b[s] = nb.d[kNbr - 1] < kInfF ? sqrt((double)nb.d[kNbr - 1]) * (1.0 - 1e-6) - 4e-3 + disp : (double)kInfF;
+    if (rest < 0.0f) rest = nb.d[kNbr - 1];
+    if (gl == 0) P.nbr_b[s] = rest < kInfF ? sqrt((double)rest) * (1.0 - 1e-6) - 4e-3 + disp : (double)kInfF;
   }
   // E-step: candidate j = gl + G q on its lane (its voxel count: 0 for an invalid range, which
   // flags the frame)
@@ -956,7 +1086,11 @@ __global__ void __launch_bounds__(kKnnWarps * 32, kKnnBlocks) k_knn_estep(DevPla
   const int gl = lane & (G - 1), gbase = lane - gl;
   const unsigned gmask = G == 32 ? 0xffffffffu : ((1u << G) - 1u) << gbase;
   const int s = blockIdx.x * (kKnnWarps * 32 / G) + (threadIdx.x >> 5) * (32 / G) + gbase / G;
-  knn_estep_sv<G>(P, s, P.iter, gl, gbase, gmask);
+  // the group's shared scratch of a search (see knn_group_collect)
+  __shared__ float2 s_keep[kKnnWarps * 32 / G][kKnnKeep + kNbr];
+  __shared__ int s_count[kKnnWarps * 32 / G];
+  const int grp = threadIdx.x / G;
+  knn_estep_sv<G>(P, s, P.iter, gl, gbase, gmask, s_keep[grp], &s_count[grp]);
 }
 
 // M-step contribution of one (supervoxel, slot) pair to Gaussian k, moments re-centred
@@ -2446,7 +2580,7 @@ __global__ void __launch_bounds__(kLSWarps * 32, kLSBlocks) k_ll_stream(DevPlan 
       if (item < knn_items) {
         const int gl = lane & (G - 1), gbase = lane - gl;
         const unsigned gmask = G == 32 ? 0xffffffffu : ((1u << G) - 1u) << gbase;
-        knn_estep_sv<G>(P, item * kPerItem + gbase / G, P.iter + 1, gl, gbase, gmask);
+        knn_estep_sv<G>(P, item * kPerItem + gbase / G, P.iter + 1, gl, gbase, gmask, nullptr, nullptr);
         __syncwarp();
       } else {
         knn_more = false;
@@ -3068,42 +3202,6 @@ __global__ void __launch_bounds__(256) k_sa_fill(const float* __restrict__ ref, 
   w.refs[w.start[p.x] + p.y] = make_float4(rk[0], rk[comp], rk[2 * comp], __int_as_float(k));
 }
 
-// Where a query sits in the grid: its cell, the gaps to that cell's faces, and the float
-// rounding of the scaled coordinates and faces (eps0; distances of d add 1e-6 d).
-struct SaPlace {
-  int c[3];
-  float f0[3], f1[3];  // gaps to the cell's lower and upper faces
-  float delta, eps0;   // the smallest gap; the rounding
-  __device__ __forceinline__ SaPlace(float q0, float q1, float q2, const float* s, const GridGeom& g) {
-    const float y[3] = {q0 * s[0], q1 * s[1], q2 * s[2]};
-    float ymax = 0.0f;
-    delta = kInfF;
-#pragma unroll
-    for (int a = 0; a < 3; a++) {
-      c[a] = cell_coord(y[a], g.lo[a], g.inv_h, g.dims[a]);
-      f0[a] = y[a] - (g.lo[a] + c[a] * g.h);
-      f1[a] = (g.lo[a] + (c[a] + 1) * g.h) - y[a];
-      delta = fminf(delta, fminf(f0[a], f1[a]));
-      ymax = fmaxf(ymax, fabsf(y[a]));
-    }
-    delta = fmaxf(delta, 0.0f);
-    eps0 = 4e-3f + 1e-6f * ymax;
-  }
-  // A squared distance below which every reference lies in the cells at Chebyshev distance
-  // <= r (0: none is known).  References outside the box sit in the boundary cells, farther
-  // from a query inside it than those cells.
-  __device__ __forceinline__ float bound2(int r, float h) const {
-    const float lb = r * h + delta, m = lb - (eps0 + 1e-6f * lb);
-    return m > 0.0f ? m * m : 0.0f;
-  }
-  // squared lower bound of the distance along axis a to the cells at offset o
-  __device__ __forceinline__ float gap2(int a, int o, float h) const {
-    const float gap = o < 0 ? f0[a] + (float)(-o - 1) * h : f1[a] + (float)(o - 1) * h;
-    const float m = fmaxf(gap - eps0 - 1e-6f * gap, 0.0f);
-    return o == 0 ? 0.0f : m * m;
-  }
-};
-
 template <typename F>
 __device__ __forceinline__ void sa_scan_cell(const SaScratch& w, int cell, float q0, float q1, float q2, const float* s,
                                              F take) {
@@ -3120,7 +3218,7 @@ __device__ __forceinline__ void sa_scan_cell(const SaScratch& w, int cell, float
 template <int N>
 __device__ __noinline__ void sa_search_thread(float q0, float q1, float q2, const float* s, const GridGeom& g,
                                               const SaScratch& w, TopN<N>& best) {
-  const SaPlace p(q0, q1, q2, s, g);
+  const GridPlace p(q0, q1, q2, s, g);
   topn_init<N>(best);
   const int maxr = max(g.dims[0], max(g.dims[1], g.dims[2]));
   for (int r = 0; r <= maxr; ++r) {
@@ -3151,7 +3249,7 @@ __device__ __noinline__ void sa_search_thread(float q0, float q1, float q2, cons
 template <int G, int N>
 __device__ __noinline__ void sa_search_group(float q0, float q1, float q2, const float* s, const GridGeom& g,
                                              const SaScratch& w, TopN<N>& best, int gl, unsigned gmask) {
-  const SaPlace p(q0, q1, q2, s, g);
+  const GridPlace p(q0, q1, q2, s, g);
   topn_init<N>(best);
   const int maxr = max(1, max(g.dims[0], max(g.dims[1], g.dims[2])));
   for (int r = 1; r <= maxr; ++r) {
