@@ -12,11 +12,15 @@
 //                in ascending linear index (ballot + popcount: no sort), with their values;
 //   k_fb_trim    a block per supervoxel: the trimming threshold (two order statistics by a
 //                two-pass radix select over 256-bin histograms, Otsu's threshold), the
-//                flood from the brightest voxel (level-synchronous; candidate and reached
-//                bits of the supervoxel's box in shared memory, or one bit per volume voxel
-//                in global memory for boxes beyond 65536 voxels), each list entry's verdict,
-//                and for kept supervoxels the FP32 centroid in the reference's summation
-//                order and the range of the background-subtracted values;
+//                flood from the brightest voxel (rows of the box as words in shared memory,
+//                swept until nothing changes; level by level from a queue where the box is wider
+//                than 32, touches an x or y border or exceeds 65536 voxels, the last with one bit
+//                per volume voxel in global memory), each list entry's verdict, and for kept
+//                supervoxels the FP32 centroid in the reference's summation order and the range
+//                of the background-subtracted values.  20,019 supervoxels of 14.5 M voxels:
+//                1049 us with the queue for all and a warp's centroid over every voxel, 433 us;
+//                bound by each block's chain of barriers, seven blocks an SM (five at 48
+//                registers 490, six 460, eight 433);
 //   k_fb_order   one block: the reference's erase order (a closed form of its
 //                swap-to-the-back loop, resolved by pointer jumping), the [0,1] rescale
 //                factors;
@@ -35,6 +39,7 @@ namespace {
 
 constexpr int kFbMaxOff = 74;
 constexpr int kFbTrimThreads = 256;  // also the Otsu histogram's bins: a thread per bin
+constexpr int kFbGroupRows = 8;  // rows of a box in flight per warp of the grouping
 constexpr int kFbScanDepth = 4;  // 16-byte label groups each lane of the scan has in flight
 
 struct FbBox {
@@ -45,6 +50,7 @@ struct FbOffsets {
   int64_t off[kFbMaxOff];    // linear-index offsets, as the reference builds them
   int8_t d[kFbMaxOff][3];    // their (dx, dy, dz)
   int32_t n;
+  int32_t rz, rxy, faces;    // reach along z and in the plane; faces only
   // unsigned division of a 32-bit linear index by X and by X*Y as a multiply-high and shifts
   // (Granlund and Montgomery's method; exact for every 32-bit numerator)
   uint32_t mx, mxy;
@@ -63,6 +69,13 @@ void div_magic(uint32_t d, uint32_t* m, int32_t* l) {
 __device__ __forceinline__ uint32_t div_by_magic(uint32_t n, uint32_t m, int32_t l) {
   const uint32_t t = __umulhi(n, m);
   return l == 0 ? n : (t + ((n - t) >> 1)) >> (l - 1);
+}
+
+// A linear index's coordinates, with the precomputed divisions of `o`.
+__device__ __forceinline__ void decode(uint32_t v, uint32_t X, uint32_t XY, const FbOffsets& o, int32_t* x,
+                                       int32_t* y, int32_t* z) {
+  const uint32_t zz = div_by_magic(v, o.mxy, o.lxy), r = v - zz * XY, yy = div_by_magic(r, o.mx, o.lx);
+  *x = (int32_t)(r - yy * X), *y = (int32_t)yy, *z = (int32_t)zz;
 }
 
 // per-call scalars shared by the kernels
@@ -147,6 +160,18 @@ __global__ void __launch_bounds__(256) k_fb_init(int32_t n, FbWork w) {
   }
 }
 
+// The box grown to hold an extent.  (Reading the bounds first and leaving out the atomics that
+// change nothing was slower: the scan is bound by issue, not by its atomics.)
+__device__ __forceinline__ void grow_box(FbBox* b, int32_t x0, int32_t x1, int32_t y0, int32_t y1, int32_t z0,
+                                         int32_t z1) {
+  atomicMin(&b->lo[0], x0);
+  atomicMax(&b->hi[0], x1);
+  atomicMin(&b->lo[1], y0);
+  atomicMax(&b->hi[1], y1);
+  atomicMin(&b->lo[2], z0);
+  atomicMax(&b->hi[2], z1);
+}
+
 // One label of the scan: its lanes (those that matched) add their count and extent once.
 __device__ __forceinline__ void scan_label(uint32_t l, uint32_t v, uint32_t X, uint32_t XY, int32_t n, int lane,
                                            FbWork& w) {
@@ -161,14 +186,8 @@ __device__ __forceinline__ void scan_label(uint32_t l, uint32_t v, uint32_t X, u
   const int32_t z0 = (int32_t)__reduce_min_sync(m, z), z1 = (int32_t)__reduce_max_sync(m, z);
   if (l != 0 && (m & ((1u << lane) - 1u)) == 0) {
     const int s = (int)l - 1;
-    FbBox* b = &w.box[s];
     atomicAdd(&w.cnt[s], __popc(m));
-    atomicMin(&b->lo[0], x0);
-    atomicMax(&b->hi[0], x1);
-    atomicMin(&b->lo[1], y0);
-    atomicMax(&b->hi[1], y1);
-    atomicMin(&b->lo[2], z0);
-    atomicMax(&b->hi[2], z1);
+    grow_box(&w.box[s], x0, x1, y0, y1, z0, z1);
   }
 }
 
@@ -177,8 +196,13 @@ __device__ __forceinline__ void scan_label(uint32_t l, uint32_t v, uint32_t X, u
 // warp holding the same label combine theirs (match, reductions) and one of them adds the sums
 // into the supervoxel's count and box.  Neighbouring voxels almost always share a label, so a
 // warp usually takes one round for its 128 voxels.
+// Where the warp's 128 voxels lie in one row, the labels are taken from the whole warp one after
+// the other: four ballots give a label's count and extent along x, the row gives the rest, and
+// seven lanes add to the count and box at once (537 M labels, a quarter of the groups labelled:
+// 95 warp instructions a group of 128 with matches and reductions for every label, the scan
+// bound by issue at 542 us; 66 and 392 us this way, 5.5 TB/s).
 __device__ __forceinline__ void scan_group(uint4 q, uint32_t v, uint32_t X, uint32_t XY, int32_t n, int lane,
-                                           FbWork& w) {
+                                           const FbOffsets& off, FbWork& w) {
   uint32_t l[4] = {q.x, q.y, q.z, q.w};
   bool bad = false;
 #pragma unroll
@@ -188,6 +212,31 @@ __device__ __forceinline__ void scan_group(uint4 q, uint32_t v, uint32_t X, uint
       l[i] = 0;
     }
   if (bad) atomicOr(&w.stat->flags, 1u);
+  int32_t xf, yf, zf;
+  decode(v - 4 * lane, X, XY, off, &xf, &yf, &zf);  // the warp's first voxel
+  if ((uint32_t)xf + 127 < X) {
+    while (true) {
+      const uint32_t first = l[0] ? l[0] : l[1] ? l[1] : l[2] ? l[2] : l[3];
+      const unsigned some = __ballot_sync(0xffffffffu, first != 0);
+      if (some == 0) return;
+      const uint32_t cur = __shfl_sync(0xffffffffu, first, __ffs(some) - 1);
+      unsigned m[4];
+#pragma unroll
+      for (int i = 0; i < 4; i++) {
+        m[i] = __ballot_sync(0xffffffffu, l[i] == cur);
+        if (l[i] == cur) l[i] = 0;
+      }
+      const unsigned any = m[0] | m[1] | m[2] | m[3];
+      const int a = __ffs(any) - 1, e = 31 - __clz(any);
+      const int x0 = xf + 4 * a + ((m[0] >> a) & 1 ? 0 : (m[1] >> a) & 1 ? 1 : (m[2] >> a) & 1 ? 2 : 3);
+      const int x1 = xf + 4 * e + ((m[3] >> e) & 1 ? 3 : (m[2] >> e) & 1 ? 2 : (m[1] >> e) & 1 ? 1 : 0);
+      const int s = (int)cur - 1;
+      FbBox* b = &w.box[s];
+      if (lane < 3) atomicMin(&b->lo[lane], lane == 0 ? x0 : lane == 1 ? yf : zf);
+      if (lane < 3) atomicMax(&b->hi[lane], lane == 0 ? x1 : lane == 1 ? yf : zf);
+      if (lane == 3) atomicAdd(&w.cnt[s], __popc(m[0]) + __popc(m[1]) + __popc(m[2]) + __popc(m[3]));
+    }
+  }
   const uint32_t z = v / XY, r = v - z * XY, y = r / X, x = r - y * X;
   while (true) {
     const uint32_t cur = l[0] ? l[0] : l[1] ? l[1] : l[2] ? l[2] : l[3];
@@ -225,14 +274,8 @@ __device__ __forceinline__ void scan_group(uint4 q, uint32_t v, uint32_t X, uint
     z1 = __reduce_max_sync(m, z1);
     if (cur != 0 && (m & ((1u << lane) - 1u)) == 0) {
       const int s = (int)cur - 1;
-      FbBox* b = &w.box[s];
       atomicAdd(&w.cnt[s], cnt);
-      atomicMin(&b->lo[0], x0);
-      atomicMax(&b->hi[0], x1);
-      atomicMin(&b->lo[1], y0);
-      atomicMax(&b->hi[1], y1);
-      atomicMin(&b->lo[2], z0);
-      atomicMax(&b->hi[2], z1);
+      grow_box(&w.box[s], x0, x1, y0, y1, z0, z1);
     }
   }
 }
@@ -241,7 +284,7 @@ __device__ __forceinline__ void scan_group(uint4 q, uint32_t v, uint32_t X, uint
 // labels are all 0 (most of a volume) do nothing more.  Coordinates in 32-bit arithmetic
 // (X*Y*Z < 2^32).
 __global__ void __launch_bounds__(256) k_fb_scan(const uint32_t* __restrict__ label, int64_t nvol, int32_t X,
-                                                 int32_t Y, int32_t n, FbWork w) {
+                                                 int32_t Y, int32_t n, FbOffsets off, FbWork w) {
   const int lane = threadIdx.x & 31;
   const uint32_t XY = (uint32_t)X * (uint32_t)Y;
   const int64_t nq = nvol / 4;  // whole 16-byte groups
@@ -260,7 +303,7 @@ __global__ void __launch_bounds__(256) k_fb_scan(const uint32_t* __restrict__ la
     for (int u = 0; u < kFbScanDepth; u++) {
       if (__ballot_sync(0xffffffffu, (q[u].x | q[u].y | q[u].z | q[u].w) != 0) == 0) continue;
       const uint32_t v = (uint32_t)(4 * (base + u * G + lane));
-      scan_group(q[u], v, X, XY, n, lane, w);
+      scan_group(q[u], v, X, XY, n, lane, off, w);
     }
   }
   if (blockIdx.x == 0 && threadIdx.x < 32) {  // the last nvol % 4 labels
@@ -278,7 +321,8 @@ __device__ T block_scan_1024(int32_t n, F count, T* out) {
   const int per = (n + 1023) / 1024;
   const int a = min(n, t * per), b = min(n, a + per);
   T sum = 0;
-  for (int i = a; i < b; i++) sum += count(i);
+#pragma unroll 8
+  for (int i = a; i < b; i++) sum += count(i);  // independent loads, eight in flight
   part[t] = sum;
   __syncthreads();
   for (int o = 1; o < 1024; o <<= 1) {
@@ -288,9 +332,11 @@ __device__ T block_scan_1024(int32_t n, F count, T* out) {
     __syncthreads();
   }
   T run = part[t] - sum;
+#pragma unroll 8
   for (int i = a; i < b; i++) {
+    const T c = count(i);
     out[i] = run;
-    run += count(i);
+    run += c;
   }
   const T total = part[1023];
   __syncthreads();
@@ -312,27 +358,35 @@ __global__ void __launch_bounds__(256) k_fb_group(const uint32_t* __restrict__ l
   int64_t at = w.uptr[s];
   if (at == w.uptr[s + 1]) return;  // no voxels: no box
   const unsigned below = (1u << lane) - 1u;
-  if (bx.hi[0] - bx.lo[0] < 32) {  // one chunk per row: four rows' labels in flight
-    const int32_t x = bx.lo[0] + lane;
+  if (bx.hi[0] - bx.lo[0] < 32) {
+    // one chunk per row: kFbGroupRows rows' labels in flight, then their voxels' values (four
+    // rows at a time, with each value loaded where it is stored: 310 us on 10,000 supervoxels;
+    // 178 us with eight, 209 with four, 183 with sixteen)
+    const int32_t x = bx.lo[0] + lane, bh = bx.hi[1] - bx.lo[1] + 1;
     const bool xin = x <= bx.hi[0];
-    for (int32_t z = bx.lo[2]; z <= bx.hi[2]; z++)
-      for (int32_t y = bx.lo[1]; y <= bx.hi[1]; y += 4) {
-        uint32_t l[4];
+    const int32_t rows = bh * (bx.hi[2] - bx.lo[2] + 1);
+    for (int32_t r0 = 0; r0 < rows; r0 += kFbGroupRows) {
+      uint32_t l[kFbGroupRows], v[kFbGroupRows];
+      uint16_t val[kFbGroupRows];
 #pragma unroll
-        for (int u = 0; u < 4; u++)
-          l[u] = (xin && y + u <= bx.hi[1]) ? label[((int64_t)z * Y + y + u) * X + x] : 0u;
-#pragma unroll
-        for (int u = 0; u < 4; u++) {
-          const bool in = l[u] == want;
-          const unsigned m = __ballot_sync(0xffffffffu, in);
-          if (in) {
-            const int64_t p = at + __popc(m & below), v = ((int64_t)z * Y + y + u) * X + x;
-            w.ulin[p] = (uint32_t)v;
-            w.uval[p] = raw[v];
-          }
-          at += __popc(m);
-        }
+      for (int u = 0; u < kFbGroupRows; u++) {
+        const int32_t r = r0 + u, z = bx.lo[2] + r / bh, y = bx.lo[1] + r % bh;
+        v[u] = (uint32_t)(((int64_t)z * Y + y) * X + x);
+        l[u] = xin && r < rows ? label[v[u]] : 0u;
       }
+#pragma unroll
+      for (int u = 0; u < kFbGroupRows; u++) val[u] = l[u] == want ? raw[v[u]] : (uint16_t)0;
+#pragma unroll
+      for (int u = 0; u < kFbGroupRows; u++) {
+        const unsigned m = __ballot_sync(0xffffffffu, l[u] == want);
+        if (l[u] == want) {
+          const int64_t p = at + __popc(m & below);
+          w.ulin[p] = v[u];
+          w.uval[p] = val[u];
+        }
+        at += __popc(m);
+      }
+    }
     if (lane == 0 && at != w.uptr[s + 1]) atomicOr(&w.stat->flags, 4u);  // box and count disagree
     return;
   }
@@ -357,7 +411,7 @@ __global__ void __launch_bounds__(256) k_fb_group(const uint32_t* __restrict__ l
 // List form: a warp per supervoxel checks its list (ascending linear indices inside the
 // volume; else the lists are flagged inconsistent) and takes its count and box.
 __global__ void __launch_bounds__(256) k_fbl_boxes(int32_t X, int32_t Y, int64_t nvol, int64_t n_list, int32_t n,
-                                                   FbWork w) {
+                                                   FbOffsets off, FbWork w) {
   const int lane = threadIdx.x & 31;
   const int s = (int)((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5);
   if (s >= n) return;
@@ -372,15 +426,30 @@ __global__ void __launch_bounds__(256) k_fbl_boxes(int32_t X, int32_t Y, int64_t
   const uint32_t XY = (uint32_t)X * (uint32_t)Y;
   int32_t lo[3] = {0x7fffffff, 0x7fffffff, 0x7fffffff}, hi[3] = {-1, -1, -1};
   bool bad = false;
-  for (int64_t i = a + lane; i < b; i += 32) {
-    const uint32_t v = w.ulin[i];
-    bad |= (int64_t)v >= nvol || (i > a && w.ulin[i - 1] >= v);
-    const uint32_t zz = v / XY, r = v - zz * XY, yy = r / (uint32_t)X;
-    const int32_t c[3] = {(int32_t)(r - yy * (uint32_t)X), (int32_t)yy, (int32_t)zz};
+  uint32_t last = 0;  // the entry before this group of 32 (lane 31's)
+  // the divisions by X and X*Y as multiplies and four groups of 32 entries in flight: 14.5 M
+  // entries 75 -> 46 us
+  for (int64_t i0 = a; i0 < b; i0 += 128) {
+    uint32_t v[4];
 #pragma unroll
-    for (int d = 0; d < 3; d++) {
-      lo[d] = min(lo[d], c[d]);
-      hi[d] = max(hi[d], c[d]);
+    for (int u = 0; u < 4; u++) {
+      const int64_t i = i0 + 32 * u + lane;
+      v[u] = i < b ? w.ulin[i] : 0u;
+    }
+#pragma unroll
+    for (int u = 0; u < 4; u++) {
+      const int64_t i = i0 + 32 * u + lane;
+      const uint32_t up = __shfl_up_sync(0xffffffffu, v[u], 1), prev = lane == 0 ? last : up;
+      last = __shfl_sync(0xffffffffu, v[u], 31);
+      if (i >= b) continue;
+      bad |= (int64_t)v[u] >= nvol || (i > a && prev >= v[u]);
+      int32_t c[3];
+      decode(v[u], (uint32_t)X, XY, off, &c[0], &c[1], &c[2]);
+#pragma unroll
+      for (int d = 0; d < 3; d++) {
+        lo[d] = min(lo[d], c[d]);
+        hi[d] = max(hi[d], c[d]);
+      }
     }
   }
   const bool any_bad = __any_sync(0xffffffffu, bad);
@@ -430,15 +499,21 @@ __device__ void warp_hist_select(const int32_t* h, int32_t k, int32_t* bucket, i
 
 constexpr int kFbMaskWords = 2048;  // bounding boxes up to 65536 voxels flood in shared memory
 
-// A linear index's coordinates, with the precomputed divisions of `o`.
-__device__ __forceinline__ void decode(uint32_t v, uint32_t X, uint32_t XY, const FbOffsets& o, int32_t* x,
-                                       int32_t* y, int32_t* z) {
-  const uint32_t zz = div_by_magic(v, o.mxy, o.lxy), r = v - zz * XY, yy = div_by_magic(r, o.mx, o.lx);
-  *x = (int32_t)(r - yy * X), *y = (int32_t)yy, *z = (int32_t)zz;
+// The bits of `cand` joined to those of `g` by runs of `cand` along the word, both ways.
+__device__ __forceinline__ uint32_t fill_runs(uint32_t g, uint32_t cand) {
+  uint32_t up = g, pu = cand, dn = g, pd = cand;
+#pragma unroll
+  for (int k = 1; k < 32; k <<= 1) {
+    up |= pu & (up << k);
+    pu &= pu << k;
+    dn |= pd & (dn >> k);
+    pd &= pd >> k;
+  }
+  return up | dn;
 }
 
 template <bool kLists>
-__global__ void __launch_bounds__(kFbTrimThreads) k_fb_trim(const uint32_t* __restrict__ label,
+__global__ void __launch_bounds__(kFbTrimThreads, 7) k_fb_trim(const uint32_t* __restrict__ label,
                                                             const uint16_t* __restrict__ raw, int64_t nvol,
                                                             int32_t X, int32_t Y, int32_t Z, int32_t n,
                                                             int32_t max_size, float max_pct, int32_t min_size,
@@ -446,7 +521,7 @@ __global__ void __launch_bounds__(kFbTrimThreads) k_fb_trim(const uint32_t* __re
   __shared__ int32_t h_hi[256], h_lo1[256], h_lo2[256], h_ot[256];
   __shared__ float s_sumb[256];
   __shared__ int32_t s_wb[256];
-  __shared__ uint32_t s_min, s_max, s_seed, s_tail;
+  __shared__ uint32_t s_min, s_max, s_min2, s_max2, s_seed, s_tail;
   __shared__ int32_t s_b1, s_r1, s_b2, s_r2, s_l1, s_l2, s_rr, s_best;
   __shared__ float s_mm;
   __shared__ uint32_t s_cand[kFbMaskWords], s_reach[kFbMaskWords];
@@ -470,8 +545,8 @@ __global__ void __launch_bounds__(kFbTrimThreads) k_fb_trim(const uint32_t* __re
   h_lo2[t] = 0;
   h_ot[t] = 0;
   if (t == 0) {
-    s_min = 0xffffffffu;
-    s_max = 0;
+    s_min = s_min2 = 0xffffffffu;
+    s_max = s_max2 = 0;
     s_seed = 0xffffffffu;
     s_tail = 0;
     s_b1 = s_b2 = 255;
@@ -608,8 +683,70 @@ __global__ void __launch_bounds__(kFbTrimThreads) k_fb_trim(const uint32_t* __re
   const FbBox bx = w.box[s];
   const int32_t bw = bx.hi[0] - bx.lo[0] + 1, bh = bx.hi[1] - bx.lo[1] + 1, bd = bx.hi[2] - bx.lo[2] + 1;
   const bool shared_path = (int64_t)bw * bh * bd <= 32 * kFbMaskWords;
+  // A box at most 32 wide, clear of the x and y borders (no offset wraps), floods a row of voxels
+  // at a time, a word per row: each sweep joins every row with its neighbour rows and fills it
+  // along x, in place, until nothing changes.  The connected set is the queue's; some ten sweeps
+  // of one barrier took the place of some 25 levels of two barriers, a decode per voxel and an
+  // atomic per neighbour (half the kernel's time).
+  const bool row_path = shared_path && bw <= 32 && bh * bd <= kFbMaskWords && bx.lo[0] >= off.rxy &&
+                        bx.hi[0] < X - off.rxy && bx.lo[1] >= off.rxy && bx.hi[1] < Y - off.rxy;
+  // a voxel's word and bit in the masks of the row path
+  auto row_of = [&](uint32_t v, uint32_t* bit) {
+    int32_t x, y, z;
+    decode(v, uX, XY, off, &x, &y, &z);
+    *bit = 1u << (x - bx.lo[0]);
+    return (y - bx.lo[1]) + bh * (z - bx.lo[2]);
+  };
   uint32_t* q = w.queue + a;
-  if (shared_path) {
+  if (row_path) {
+    const int32_t rows = bh * bd;
+    for (int i = t; i < rows; i += kFbTrimThreads) s_cand[i] = s_reach[i] = 0u;
+    __syncthreads();
+    for (int32_t i = t; i < N; i += kFbTrimThreads)
+      if (val[i] > th) {
+        uint32_t bit;
+        const int32_t r = row_of(lin[i], &bit);
+        atomicOr(&s_cand[r], bit);
+        if ((uint32_t)i == s_seed) s_reach[r] = bit;  // one entry; no other thread writes reach yet
+      }
+    __syncthreads();
+    volatile uint32_t* reach = s_reach;
+    for (;;) {
+      int changed = 0;
+      for (int32_t r = t; r < rows; r += kFbTrimThreads) {
+        const uint32_t cand = s_cand[r], cur = reach[r];
+        if (cur == cand) continue;
+        const int32_t z = r / bh, y = r - z * bh;
+        uint32_t nb = cur;
+        if (off.faces) {
+          if (y > 0) nb |= reach[r - 1];
+          if (y < bh - 1) nb |= reach[r + 1];
+          if (off.rz) {
+            if (z > 0) nb |= reach[r - bh];
+            if (z < bd - 1) nb |= reach[r + bh];
+          }
+        } else {
+          for (int dz = -off.rz; dz <= off.rz; dz++)
+            for (int dy = -off.rxy; dy <= off.rxy; dy++) {
+              if (z + dz < 0 || z + dz >= bd || y + dy < 0 || y + dy >= bh) continue;
+              const uint32_t m = reach[r + dy + bh * dz];
+              nb |= m | m << 1 | m >> 1;
+              if (off.rxy == 2) nb |= m << 2 | m >> 2;
+            }
+        }
+        const uint32_t now = fill_runs(nb & cand, cand);
+        if (now != cur) {
+          reach[r] = now;
+          changed = 1;
+        }
+      }
+      if (!__syncthreads_or(changed)) break;
+    }
+    int32_t mine = 0;
+    for (int32_t r = t; r < rows; r += kFbTrimThreads) mine += __popc(s_reach[r]);
+    mine = __reduce_add_sync(0xffffffffu, mine);
+    if (lane == 0 && mine) atomicAdd(&s_tail, (uint32_t)mine);
+  } else if (shared_path) {
     const int32_t words = (bw * bh * bd + 31) / 32;
     for (int i = t; i < words; i += kFbTrimThreads) s_cand[i] = s_reach[i] = 0u;
     __syncthreads();
@@ -629,15 +766,21 @@ __global__ void __launch_bounds__(kFbTrimThreads) k_fb_trim(const uint32_t* __re
       q[0] = lin[s_seed];
       s_tail = 1;
     }
-  } else if (t == 0 && val[s_seed] > th) {
-    const uint32_t v = lin[s_seed];
-    atomicOr(&w.bits[v >> 5], 1u << (v & 31));
-    q[0] = v;
-    s_tail = 1;
+  } else {
+    // the supervoxel's own voxels' bits (those the flood tests and sets) start clear; a word may
+    // hold another's, whose block does the same
+    for (int32_t i = t; i < N; i += kFbTrimThreads) atomicAnd(&w.bits[lin[i] >> 5], ~(1u << (lin[i] & 31)));
+    __syncthreads();
+    if (t == 0 && val[s_seed] > th) {
+      const uint32_t v = lin[s_seed];
+      atomicOr(&w.bits[v >> 5], 1u << (v & 31));
+      q[0] = v;
+      s_tail = 1;
+    }
   }
   __syncthreads();
   const uint32_t want = (uint32_t)s + 1u;
-  uint32_t head = 0;
+  uint32_t head = row_path ? s_tail : 0;  // (the row path has nothing queued)
   for (;;) {
     const uint32_t tail = s_tail;
     __syncthreads();
@@ -694,79 +837,85 @@ __global__ void __launch_bounds__(kFbTrimThreads) k_fb_trim(const uint32_t* __re
   }
   const int32_t kept = (int32_t)s_tail;
   // each list entry's verdict, for the centroid and the emission
-  for (int32_t i = t; i < N; i += kFbTrimThreads) {
-    const uint32_t v = lin[i];
-    bool in;
+  auto verdict = [&](uint32_t v) -> bool {
+    if (row_path) {
+      uint32_t bit;
+      const int32_t r = row_of(v, &bit);
+      return (s_reach[r] & bit) != 0;
+    }
     if (shared_path) {
       int32_t x, y, z;
       decode(v, uX, XY, off, &x, &y, &z);
       const int32_t li = (x - bx.lo[0]) + bw * ((y - bx.lo[1]) + bh * (z - bx.lo[2]));
-      in = (s_reach[li >> 5] >> (li & 31)) & 1u;
-    } else {  // the flood's bits were set by atomics at L2: read them there
-      in = (__ldcg(&w.bits[v >> 5]) >> (v & 31)) & 1u;
+      return (s_reach[li >> 5] >> (li & 31)) & 1u;
     }
-    keep[i] = in ? 1 : 0;
-  }
+    // the flood's bits were set by atomics at L2: read them there
+    return (__ldcg(&w.bits[v >> 5]) >> (v & 31)) & 1u;
+  };
   if (t == 0) w.tcnt[s] = kept;
-  if (kept < min_size) return;
-  __syncthreads();
-  if (t >= 32) return;
-  // warp 0: the centroid in list order (FP32, as the reference sums it) and the range of the
-  // background-subtracted values.  Each lane forms its voxel's products and stages them (zeros
-  // for a voxel not kept: every term is non-negative, so adding +0 leaves a sum's bits as they
-  // are); the four running sums then add the group's 32 entries in lane order (list order), from
-  // broadcast loads issued ahead of the additions, so the chains hold only the additions.
-  __shared__ float4 st4[32];
-  float sw = 0.0f, c0 = 0.0f, c1 = 0.0f, c2 = 0.0f;
+  if (kept < min_size) {  // erased: its verdicts are not read
+    return;
+  }
+  // The centroid in list order (FP32, as the reference sums it) and the range of the
+  // background-subtracted values.  The block forms the kept voxels' products 256 list entries at
+  // a time and packs them in list order; four lanes then add them one after the other, a running
+  // sum each, so that the serial part holds one load and one addition per kept voxel (a voxel not
+  // kept would add +0 to non-negative sums and leave their bits).
+  __shared__ float4 s_prod[kFbTrimThreads];
+  __shared__ int32_t s_wn[kFbTrimThreads / 32];
+  float acc = 0.0f;  // lanes 0-3 of warp 0: I, I x, I y, I z
   uint32_t smin = 0xffffffffu, smax = 0;
-  for (int32_t i0 = 0; i0 < N; i0 += 32) {
-    const int32_t i = i0 + lane;
+  for (int32_t i0 = 0; i0 < N; i0 += kFbTrimThreads) {
+    const int32_t i = i0 + t;
     bool in = false;
     uint32_t v = 0, r = 0;
     if (i < N) {
       v = lin[i];
       r = val[i];
-      in = keep[i] != 0;
+      in = verdict(v);
+      keep[i] = in ? 1 : 0;
     }
     const unsigned m = __ballot_sync(0xffffffffu, in);
-    float I = 0.0f, px = 0.0f, py = 0.0f, pz = 0.0f;
+    if (lane == 0) s_wn[t >> 5] = __popc(m);
+    __syncthreads();
+    int32_t at = __popc(m & ((1u << lane) - 1u)), n_in = 0;
+#pragma unroll
+    for (int k = 0; k < kFbTrimThreads / 32; k++) {
+      if (k < (t >> 5)) at += s_wn[k];
+      n_in += s_wn[k];
+    }
     if (in) {
       int32_t x, y, z;
       decode(v, uX, XY, off, &x, &y, &z);
-      I = (float)r;
-      px = __fmul_rn(I, (float)x);
-      py = __fmul_rn(I, (float)y);
-      pz = __fmul_rn(I, (float)z);
+      const float I = (float)r;
+      s_prod[at] = make_float4(I, __fmul_rn(I, (float)x), __fmul_rn(I, (float)y), __fmul_rn(I, (float)z));
       const uint32_t sub = (uint16_t)(r - th);
       smin = min(smin, sub);
       smax = max(smax, sub);
     }
-    st4[lane] = make_float4(I, px, py, pz);
-    __syncwarp();
-    if (m) {
-#pragma unroll
-      for (int p = 0; p < 32; p++) {
-        const float4 e = st4[p];
-        sw = __fadd_rn(sw, e.x);
-        c0 = __fadd_rn(c0, e.y);
-        c1 = __fadd_rn(c1, e.z);
-        c2 = __fadd_rn(c2, e.w);
-      }
+    __syncthreads();
+    if (t < 4) {
+      const float* p = reinterpret_cast<const float*>(s_prod) + t;
+#pragma unroll 8
+      for (int k = 0; k < n_in; k++) acc = __fadd_rn(acc, p[4 * k]);
     }
-    __syncwarp();
   }
-  for (int o = 16; o > 0; o >>= 1) {
-    smin = min(smin, __shfl_xor_sync(0xffffffffu, smin, o));
-    smax = max(smax, __shfl_xor_sync(0xffffffffu, smax, o));
-  }
+  smin = __reduce_min_sync(0xffffffffu, smin);
+  smax = __reduce_max_sync(0xffffffffu, smax);
   if (lane == 0) {
+    atomicMin(&s_min2, smin);
+    atomicMax(&s_max2, smax);
+  }
+  __syncthreads();
+  if (t < 32) {
+    const float sw = __shfl_sync(0xffffffffu, acc, 0);
     const bool zero = (double)sw < 1e-5;
-    w.tcent[3 * s] = zero ? 0.0f : __fdiv_rn(c0, sw);
-    w.tcent[3 * s + 1] = zero ? 0.0f : __fdiv_rn(c1, sw);
-    w.tcent[3 * s + 2] = zero ? 0.0f : __fdiv_rn(c2, sw);
-    atomicMin(&w.stat->sub_min, smin);
-    atomicMax(&w.stat->sub_max, smax);
-    atomicAdd(&w.stat->kept_vox, (unsigned long long)kept);
+    if (t >= 1 && t < 4) w.tcent[3 * s + t - 1] = zero ? 0.0f : __fdiv_rn(acc, sw);
+    if (t == 0) {
+      atomicMin(&w.stat->sub_min, s_min2);
+      atomicMax(&w.stat->sub_max, s_max2);
+      atomicAdd(&w.stat->kept_vox, (unsigned long long)kept);
+    }
   }
 }
 
@@ -837,7 +986,8 @@ __global__ void __launch_bounds__(1024) k_fb_csr(int64_t max_vox, int32_t max_sv
   if (threadIdx.x == 0) lptr[S] = total;
 }
 
-__global__ void __launch_bounds__(256) k_fb_emit(int32_t X, int32_t Y, int64_t max_vox, int32_t max_sv, FbWork w,
+__global__ void __launch_bounds__(256) k_fb_emit(int32_t X, int32_t Y, int64_t max_vox, int32_t max_sv, FbOffsets off,
+                                                 FbWork w,
                                                  const int64_t* __restrict__ lptr, float* query, float* img,
                                                  float* cent, uint16_t* thr_out) {
   const FbStat* st = w.stat;
@@ -855,24 +1005,34 @@ __global__ void __launch_bounds__(256) k_fb_emit(int32_t X, int32_t Y, int64_t m
   const int32_t n = (int32_t)(w.uptr[s + 1] - a);
   int64_t at = lptr[p];
   const unsigned below = (1u << lane) - 1u;
-  for (int32_t i0 = 0; i0 < n; i0 += 32) {
-    const int32_t i = i0 + lane;
-    bool in = false;
-    uint32_t v = 0;
-    if (i < n) {
-      v = w.ulin[a + i];
-      in = w.ukeep[a + i] != 0;
+  const uint32_t XY = (uint32_t)X * (uint32_t)Y;
+  // four groups of 32 entries in flight, divisions as multiplies: 14.5 M entries 111 -> 52 us
+  for (int32_t i0 = 0; i0 < n; i0 += 128) {
+    uint32_t v[4];
+    uint16_t r[4];
+    bool in[4];
+#pragma unroll
+    for (int u = 0; u < 4; u++) {
+      const int32_t i = i0 + 32 * u + lane;
+      in[u] = i < n && w.ukeep[a + i] != 0;
+      v[u] = i < n ? w.ulin[a + i] : 0u;
+      r[u] = i < n ? w.uval[a + i] : (uint16_t)0;
     }
-    const unsigned m = __ballot_sync(0xffffffffu, in);
-    if (in) {
-      const int64_t o = at + __popc(m & below);
-      query[o] = (float)(v % (uint32_t)X);
-      query[N + o] = (float)((v / (uint32_t)X) % (uint32_t)Y);
-      query[2 * N + o] = (float)(v / ((uint32_t)X * (uint32_t)Y));
-      const float sub = (float)(uint16_t)(w.uval[a + i] - th);
-      img[o] = scaled ? (float)__dmul_rn(f, __dadd_rn((double)sub, sh)) : sub;
+#pragma unroll
+    for (int u = 0; u < 4; u++) {
+      const unsigned m = __ballot_sync(0xffffffffu, in[u]);
+      if (in[u]) {
+        const int64_t o = at + __popc(m & below);
+        int32_t x, y, z;
+        decode(v[u], (uint32_t)X, XY, off, &x, &y, &z);
+        query[o] = (float)x;
+        query[N + o] = (float)y;
+        query[2 * N + o] = (float)z;
+        const float sub = (float)(uint16_t)(r[u] - th);
+        img[o] = scaled ? (float)__dmul_rn(f, __dadd_rn((double)sub, sh)) : sub;
+      }
+      at += __popc(m);
     }
-    at += __popc(m);
   }
   if (lane == 0) {
     for (int d = 0; d < 3; d++) cent[(int64_t)d * S + p] = w.tcent[3 * s + d];
@@ -909,6 +1069,7 @@ int fb_offsets(int32_t conn, const int32_t dims[3], FbOffsets* o) {
         n++;
       }
   o->n = n;
+  o->rz = rz, o->rxy = rxy, o->faces = conn == 4 || conn == 6;
   div_magic((uint32_t)X, &o->mx, &o->lx);
   div_magic((uint32_t)XY, &o->mxy, &o->lxy);
   return n;
@@ -968,8 +1129,6 @@ int frame_build(const uint16_t* raw, const uint32_t* label, const int32_t dims[3
     if (ev) cudaEventRecord(ev[stage++], st);
   };
   mark();
-  cudaError_t e = cudaMemsetAsync(w.bits, 0, 4 * (size_t)((nvol + 31) / 32), st);
-  if (e != cudaSuccess) return report_error(TGMM_ERR_CUDA, kWhat, e);
   const unsigned warp_blocks = (unsigned)(((int64_t)n * 32 + 255) / 256);
   k_fb_init<<<(n + 255) / 256, 256, 0, st>>>(n, w);
   mark();
@@ -980,7 +1139,7 @@ int frame_build(const uint16_t* raw, const uint32_t* label, const int32_t dims[3
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_fb_scan, 256, 0);
   const int64_t span = (nvol / 4 + 256 * kFbScanDepth - 1) / (256 * kFbScanDepth);
   const int64_t full = (int64_t)sms * (occ > 0 ? occ : 1);
-  k_fb_scan<<<(unsigned)(span < 1 ? 1 : span < full ? span : full), 256, 0, st>>>(label, nvol, X, Y, n, w);
+  k_fb_scan<<<(unsigned)(span < 1 ? 1 : span < full ? span : full), 256, 0, st>>>(label, nvol, X, Y, n, off, w);
   mark();
   k_fb_ptr<<<1, 1024, 0, st>>>(n, w);
   mark();
@@ -993,10 +1152,10 @@ int frame_build(const uint16_t* raw, const uint32_t* label, const int32_t dims[3
   mark();
   k_fb_csr<<<1, 1024, 0, st>>>(max_vox, max_sv, w, lptr);
   mark();
-  k_fb_emit<<<warp_blocks, 256, 0, st>>>(X, Y, max_vox, max_sv, w, lptr, query, img, cent, thr);
+  k_fb_emit<<<warp_blocks, 256, 0, st>>>(X, Y, max_vox, max_sv, off, w, lptr, query, img, cent, thr);
   mark();
   FbStat h;
-  e = cudaGetLastError();
+  cudaError_t e = cudaGetLastError();
   if (e == cudaSuccess) e = cudaMemcpyAsync(&h, w.stat, sizeof(h), cudaMemcpyDeviceToHost, st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
   if (e != cudaSuccess) return report_error(TGMM_ERR_CUDA, kWhat, e);
@@ -1066,12 +1225,10 @@ int frame_build_lists(const uint32_t* lin, const uint16_t* val, const int64_t* l
     if (stage_ms) cudaEventRecord(evs.e[stage++], st);
   };
   mark();
-  cudaError_t e = cudaMemsetAsync(w.bits, 0, 4 * (size_t)((nvol + 31) / 32), st);
-  if (e != cudaSuccess) return report_error(TGMM_ERR_CUDA, kWhat, e);
   const unsigned warp_blocks = (unsigned)(((int64_t)n * 32 + 255) / 256);
   k_fb_init<<<(n + 255) / 256, 256, 0, st>>>(n, w);
   mark();
-  k_fbl_boxes<<<warp_blocks, 256, 0, st>>>(X, Y, nvol, n_list, n, w);
+  k_fbl_boxes<<<warp_blocks, 256, 0, st>>>(X, Y, nvol, n_list, n, off, w);
   mark();
   mark();  // no CSR to build: the lists come with theirs
   mark();  // no grouping: the lists are grouped
@@ -1082,10 +1239,10 @@ int frame_build_lists(const uint32_t* lin, const uint16_t* val, const int64_t* l
   mark();
   k_fb_csr<<<1, 1024, 0, st>>>(max_vox, max_sv, w, lptr);
   mark();
-  k_fb_emit<<<warp_blocks, 256, 0, st>>>(X, Y, max_vox, max_sv, w, lptr, query, img, cent, thr);
+  k_fb_emit<<<warp_blocks, 256, 0, st>>>(X, Y, max_vox, max_sv, off, w, lptr, query, img, cent, thr);
   mark();
   FbStat h;
-  e = cudaGetLastError();
+  cudaError_t e = cudaGetLastError();
   if (e == cudaSuccess) e = cudaMemcpyAsync(&h, w.stat, sizeof(h), cudaMemcpyDeviceToHost, st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
   if (e != cudaSuccess) return report_error(TGMM_ERR_CUDA, kWhat, e);
