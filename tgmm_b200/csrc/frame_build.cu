@@ -32,6 +32,7 @@
 #include <float.h>
 #include <stdint.h>
 
+#include "tgmm_div.cuh"
 #include "tgmm_internal.cuh"
 
 namespace tgmm {
@@ -56,20 +57,6 @@ struct FbOffsets {
   uint32_t mx, mxy;
   int32_t lx, lxy;
 };
-
-// The magic number m and the shift l of the division by d (1 <= d < 2^32): l = ceil(log2 d),
-// m = floor(2^32 (2^l - d) / d) + 1.
-void div_magic(uint32_t d, uint32_t* m, int32_t* l) {
-  int32_t k = 0;
-  while (((uint64_t)1 << k) < d) k++;
-  *m = (uint32_t)((((uint64_t)1 << 32) * (((uint64_t)1 << k) - d)) / d + 1);
-  *l = k;
-}
-
-__device__ __forceinline__ uint32_t div_by_magic(uint32_t n, uint32_t m, int32_t l) {
-  const uint32_t t = __umulhi(n, m);
-  return l == 0 ? n : (t + ((n - t) >> 1)) >> (l - 1);
-}
 
 // A linear index's coordinates, with the precomputed divisions of `o`.
 __device__ __forceinline__ void decode(uint32_t v, uint32_t X, uint32_t XY, const FbOffsets& o, int32_t* x,
