@@ -445,10 +445,10 @@ def run_ours(args):
     peak, peak_kind = measured_peaks()
     vox_bytes = 16.0 * N
     knn_bytes = 164.0 * S + 104.0 * K
-    alone = {"kernel": "k_ll_pass<0, 0, 0> (the voxel pass alone)", "ms_per_launch": ms_ll,
+    alone = {"kernel": "k_ll_stream<0> (the voxel pass alone)", "ms_per_launch": ms_ll,
              "algorithmic_bytes_per_launch": vox_bytes, "achieved": vox_bytes / (ms_ll * 1e-3) / 1e9,
              "frac": vox_bytes / (ms_ll * 1e-3) / 1e9 / peak}
-    fused = {"kernel": f"k_ll_pass<0, {max(knn_lanes, 8)}, 0> (the voxel pass running the next iteration's kNN/E-step)",
+    fused = {"kernel": f"k_ll_stream<{max(knn_lanes, 8)}> (the voxel pass running the next iteration's kNN/E-step)",
              "ms_per_launch": ms_llk, "algorithmic_bytes_per_launch": vox_bytes + knn_bytes,
              "achieved": (vox_bytes + knn_bytes) / (ms_llk * 1e-3) / 1e9,
              "frac": (vox_bytes + knn_bytes) / (ms_llk * 1e-3) / 1e9 / peak}
