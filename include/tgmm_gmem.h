@@ -410,7 +410,8 @@ enum {
 };
 int tgmm_plan_time_kernel(TgmmPlan* plan, int32_t kernel, int32_t reps, float* ms_per_launch, void* stream);
 
-/* Lanes per supervoxel of the kNN/E-step kernel (4, 8, 16 or 32; default 8; with 4 lanes a
+/* Lanes per supervoxel of the kNN/E-step kernel (4, 8, 16 or 32; until set or tuned, by the
+ * plan's capacity in supervoxels: 32 up to 1000, 16 up to 6000, 8 above; with 4 lanes a
  * lane holds two list members and lane 0 two candidates, and the kNN/E-step always runs in
  * its own kernel).  Every width computes the same bits; only the speed differs with the
  * batch (supervoxel count, cells per ring, candidates per cell).  No reference counterpart: the reference runs one fixed
@@ -418,7 +419,10 @@ int tgmm_plan_time_kernel(TgmmPlan* plan, int32_t kernel, int32_t reps, float* m
 int tgmm_plan_set_knn_group(TgmmPlan* plan, int32_t lanes);
 
 /* Whether the log-likelihood voxel pass of each iteration also runs the next iteration's
- * kNN/E-step (1) or that kernel follows the pass (0, the default).  Both give the same
+ * kNN/E-step (1) or that kernel follows the pass (0).  Until the width or this is set, or the
+ * plan tuned, a plan of up to 3000 supervoxels runs them together in calls with a fixed
+ * iteration count (a negative tolerance), every other call apart.  Setting the width alone
+ * leaves the kernels apart.  Both give the same
  * bits; running them together pays off when the voxel pass leaves the SMs idle (small
  * frames), apart when the batch is large.  No reference counterpart. */
 int tgmm_plan_set_knn_fusion(TgmmPlan* plan, int32_t on);
@@ -429,7 +433,8 @@ int tgmm_plan_set_knn_fusion(TgmmPlan* plan, int32_t on);
  * call on the plan starts from a clean state.  A short limit exercises that path. */
 int tgmm_plan_set_stage_wait(TgmmPlan* plan, int64_t wait_ns);
 
-/* The plan's current kNN/E-step width and arrangement (either pointer may be NULL). */
+/* The plan's current kNN/E-step width and arrangement (either pointer may be NULL; the
+ * arrangement of a plan neither set nor tuned is that of a fixed iteration count). */
 int tgmm_plan_tuning(TgmmPlan* plan, int32_t* lanes, int32_t* fused);
 
 /* Autotuner (no reference counterpart): runs the whole EM call of the batch (the

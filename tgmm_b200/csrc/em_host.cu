@@ -152,6 +152,21 @@ cudaError_t scratch_alloc(void** p, size_t bytes, cudaStream_t st) {
 }
 }  // namespace tgmm
 
+// A plan's kNN/E-step until it is tuned or set by hand, by its capacity in supervoxels (the
+// launches are sized by it).  The voxel pass has 2368 warps: with fewer supervoxels than that
+// the idle ones take the next iteration's kNN/E-step at once and an iteration is three kernels
+// long instead of four; wider groups shorten the chain of loads while every supervoxel still
+// fits one wave.  Twenty iterations, us, 8 lanes alone / 16 alone / 32 alone / 16 in the voxel
+// pass / 32 in it: 12 supervoxels 668 623 618 569 561; 500 837 829 806 756 741; 900 908 882 865
+// 821 795; 1200 878 846 818 776 803; 1600 908 887 857 827 855; 2500 994 970 958 943 1049; 4000
+// 1059 1044 1063 1040 1114; 7000 1299 1301 1405 1328 1469; 15000 1840 1951 2079 2143 2577.  A
+// call that stops by its tolerance drops the last kNN/E-step the voxel pass ran ahead, and gains
+// nothing from it (8, 16, 32 lanes alone and 32 in it: 300 supervoxels 382 356 332 330, 1000
+// 316 300 275 278, 5000 394 376 - 442): it keeps the kernel of its own.
+constexpr int32_t kKnnSv32 = 1000;
+constexpr int32_t kKnnSvFused = 3000;
+constexpr int32_t kKnnSv16 = 6000;
+
 struct TgmmPlan {
   TgmmPlanDesc desc;
   Layout L;
@@ -162,7 +177,10 @@ struct TgmmPlan {
   cudaEvent_t done_ev = nullptr;       // end of the last call
   cudaStream_t last_stream = nullptr;  // its stream
   bool used = false;
-  bool fuse_knn = false;  // the voxel pass runs the next iteration's kNN/E-step (autotuned)
+  bool fuse_knn = false;  // the voxel pass runs the next iteration's kNN/E-step (autotuned, set or by size)
+  // the width and the arrangement are the plan's own by size: the voxel pass runs the kNN/E-step
+  // only where the iteration count is fixed
+  bool knn_by_size = true;
   // (max_iter, ll_prec, conditional iterations) -> exec
   std::map<std::tuple<int, int, int>, cudaGraphExec_t> graphs;
   cudaStream_t fork_stream = nullptr;  // the records' branch of a call (fetch, import)
@@ -259,7 +277,8 @@ int tgmm_plan_create(const TgmmPlanDesc* d, TgmmPlan** out) {
   D.gll = (GaussLL*)(b + P->L.gll);
   D.kpos = (float4*)(b + P->L.kpos);
   D.work = (int32_t*)(b + P->L.work);
-  D.knn_group = 8;
+  D.knn_group = d->max_sv <= kKnnSv32 ? 32 : d->max_sv <= kKnnSv16 ? 16 : 8;
+  P->fuse_knn = d->max_sv <= kKnnSvFused;
   D.stage_wait_ns = 1000000000ull;
   e = configure_kernels(D, d->device);
   if (e != cudaSuccess) {
@@ -475,7 +494,7 @@ int capture_if_running(const DevPlan& D, cudaStream_t st, F body) {
 // per iteration, one after the other, spent 222 us of a 20-iteration call on a frame that
 // converged after two (a tracked step of 5000 nuclei: 641 us, 500 us this way).
 constexpr int kCondFirst = 4;  // tracked frames converge after two to four iterations
-int enqueue_em(TgmmPlan* P, int max_iter, int ll_prec, bool cond, cudaStream_t st) {
+int enqueue_em(TgmmPlan* P, int max_iter, int ll_prec, double tol, bool cond, cudaStream_t st) {
   DevPlan D = P->dev;
   D.iter = 1;
   launch_build_maps(D, st);
@@ -492,7 +511,7 @@ int enqueue_em(TgmmPlan* P, int max_iter, int ll_prec, bool cond, cudaStream_t s
   TG_CUDA(cudaStreamWaitEvent(st, P->join_ev, 0), "join");
   const bool fp64 = ll_prec == TGMM_LLPREC_FP64;
   // (the voxel pass carries the kNN/E-step in groups of 8 lanes or more)
-  const bool fuse = P->fuse_knn && !fp64 && D.knn_group >= 8;
+  const bool fuse = P->fuse_knn && !fp64 && D.knn_group >= 8 && (!P->knn_by_size || tol < 0.0);
   if (max_iter >= 1) launch_knn_estep(D, st);
   // iterations first .. last on s
   auto iterate = [&](int first, int last, cudaStream_t s) {
@@ -536,7 +555,7 @@ bool use_graphs() {
 }
 
 int run_batch(TgmmPlan* P, int max_iter, int ll_prec, double tol, cudaStream_t st) {
-  if (!use_graphs()) return enqueue_em(P, max_iter, ll_prec, false, st);
+  if (!use_graphs()) return enqueue_em(P, max_iter, ll_prec, tol, false, st);
   // a negative tolerance runs every iteration: no conditional nodes
   const bool cond = tol >= 0.0;
   auto key = std::make_tuple(max_iter, ll_prec, cond ? 1 : 0);
@@ -544,7 +563,7 @@ int run_batch(TgmmPlan* P, int max_iter, int ll_prec, double tol, cudaStream_t s
   if (it == P->graphs.end()) {
     cudaGraph_t g = nullptr;
     TG_CUDA(cudaStreamBeginCapture(P->cap_stream, cudaStreamCaptureModeThreadLocal), "begin capture");
-    int rc = enqueue_em(P, max_iter, ll_prec, cond, P->cap_stream);
+    int rc = enqueue_em(P, max_iter, ll_prec, tol, cond, P->cap_stream);
     cudaError_t e = cudaStreamEndCapture(P->cap_stream, &g);
     if (rc != TGMM_OK) {
       if (g) cudaGraphDestroy(g);
@@ -687,11 +706,13 @@ int tgmm_plan_set_knn_group(TgmmPlan* P, int32_t lanes) {
   if (lanes != 4 && lanes != 8 && lanes != 16 && lanes != 32)
     return fail(TGMM_ERR_INVALID_ARG, "tgmm_plan_set_knn_group: lanes per supervoxel must be 4, 8, 16 or 32");
   std::lock_guard<std::mutex> lock(P->mu);
-  if (P->dev.knn_group == lanes) return TGMM_OK;
+  if (P->dev.knn_group == lanes && !P->knn_by_size) return TGMM_OK;
   TG_CUDA(cudaSetDevice(P->desc.device), "cudaSetDevice");
   if (P->used) TG_CUDA(cudaEventSynchronize(P->done_ev), "wait for the previous call on this plan");
   for (auto& kv : P->graphs) cudaGraphExecDestroy(kv.second);  // captured with the old launch shape
   P->graphs.clear();
+  if (P->knn_by_size) P->fuse_knn = false;
+  P->knn_by_size = false;
   P->dev.knn_group = lanes;
   return TGMM_OK;
 }
@@ -700,11 +721,12 @@ int tgmm_plan_set_knn_fusion(TgmmPlan* P, int32_t on) {
   if (!P) return fail(TGMM_ERR_INVALID_ARG, "tgmm_plan_set_knn_fusion: null plan");
   if (on != 0 && on != 1) return fail(TGMM_ERR_INVALID_ARG, "tgmm_plan_set_knn_fusion: on must be 0 or 1");
   std::lock_guard<std::mutex> lock(P->mu);
-  if (P->fuse_knn == (on == 1)) return TGMM_OK;
+  if (P->fuse_knn == (on == 1) && !P->knn_by_size) return TGMM_OK;
   TG_CUDA(cudaSetDevice(P->desc.device), "cudaSetDevice");
   if (P->used) TG_CUDA(cudaEventSynchronize(P->done_ev), "wait for the previous call on this plan");
   for (auto& kv : P->graphs) cudaGraphExecDestroy(kv.second);  // captured with the other arrangement
   P->graphs.clear();
+  P->knn_by_size = false;
   P->fuse_knn = on == 1;
   return TGMM_OK;
 }
@@ -767,6 +789,7 @@ int tgmm_plan_autotune(TgmmPlan* P, int32_t n_frames, const TgmmFrame* frames, T
   TG_CUDA(cudaEventCreate(&ev[0]), "event");
   TG_CUDA(cudaEventCreate(&ev[1]), "event");
   const int widths[4] = {4, 8, 16, 32};
+  P->knn_by_size = false;
   float best_ms = 0.0f;
   int best_w = P->dev.knn_group;
   bool best_f = P->fuse_knn, have = false;
