@@ -263,6 +263,8 @@ __global__ void __launch_bounds__(kFrameThreads) k_build_maps(DevPlan P) {
   }
   for (int i = first; i < D.cell_budget; i += stride) P.cell_cnt[D.cell_base + i] = 0;
   if (blockIdx.y != 0) return;
+  // the voxel passes' counters, which each pass leaves at zero
+  if (f == 0 && threadIdx.x < 3) P.work[threadIdx.x] = 0;
   FrameState* S = &P.state[f];
   __shared__ float smin[3][32], smax[3][32];
   __shared__ int sbad;
@@ -327,7 +329,7 @@ __global__ void __launch_bounds__(kFrameThreads) k_build_maps(DevPlan P) {
     S->disp_cum = 0.0;
     S->disp_max = 0u;
     S->knn_searches = 0;
-    S->done = (flags & (F_BAD_CSR | F_FEW_GAUSS)) ? 1 : 0;
+    S->done = (flags & (F_BAD_CSR | F_FEW_GAUSS)) ? kNeverRan : 0;
     S->converged = 0;
     S->flags = flags;
     S->n_dead = 0;
@@ -1960,7 +1962,7 @@ __device__ void frame_converge(const DevPlan& P, int f) {
   const bool go = fabs(ll - S->ll1) / fabs(S->ll1) > D.tol && fabs(ll - S->ll2) / fabs(S->ll2) > D.tol &&
                   fabs(ll - S->ll3) / fabs(S->ll3) > D.tol;
   if (!go) S->converged = 1;
-  S->done = (!go || next > D.max_iter) ? 1 : 0;
+  S->done = (!go || next > D.max_iter) ? P.iter : 0;  // (see FrameState::done)
 }
 
 // Each warp streams the supervoxels it takes from the work counter through a ring of
@@ -2495,8 +2497,13 @@ template <int G>
 __global__ void __launch_bounds__(kLSWarps * 32, kLSBlocks) k_ll_stream(DevPlan P) {
   const int total = P.info->total_sv;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  // a lone frame that is done leaves nothing to do
-  if (P.info->n_frames == 1 && *(volatile const int32_t*)&P.state[0].done) return;
+  // A lone frame that an earlier launch ended leaves nothing to do.  One that this launch ends
+  // while a block is still waiting for a place on an SM does not count: its warps arrive at the
+  // work counters like the others, whose last one resets them.
+  if (P.info->n_frames == 1) {
+    const int done = *(volatile const int32_t*)&P.state[0].done;
+    if (done != 0 && done != P.iter) return;
+  }
   extern __shared__ __align__(128) unsigned char ll_smem[];
   LSWarp& Sh = reinterpret_cast<LSWarp*>(ll_smem)[warp];
   const unsigned ring_a = smem_addr(&Sh.ring[0][lane]);

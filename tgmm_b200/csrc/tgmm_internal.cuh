@@ -97,6 +97,7 @@ struct FrameDesc {
   int32_t max_iter, ll_mode, ll_prec, frame_id;
 };
 
+constexpr int32_t kNeverRan = -1;
 struct FrameState {
   float lo[3];
   float h;
@@ -104,6 +105,8 @@ struct FrameState {
   int32_t dims[3];
   int32_t n_cells;
   int32_t iter;  // numIterEM of the reference: the next iteration to run (starts at 1)
+  // 0 while the frame runs, then the iteration whose voxel pass ended it (kNeverRan: a frame that
+  // cannot run): a pass tells by it a frame that it ends itself from one that was over before
   int32_t done;
   int32_t converged;
   int32_t flags;
@@ -215,7 +218,9 @@ struct DevPlan {
   int32_t* nan_e;
   double* alpha_part_f;
   int32_t* dead_part;
-  int32_t* work;   // [0] next supervoxel of the voxel pass, [1] warps that left it
+  // [0] next supervoxel of the voxel pass, [1] warps that left it, [2] next kNN/E-step item of a
+  // pass that runs it; zero between launches
+  int32_t* work;
   int32_t ll_blocks;    // resident blocks of the voxel pass's FP32 forms (SMs x blocks per SM)
   int32_t ll_blocks64;  // the same for its FP64 form
   int32_t ls_blocks;    // blocks of the FP32 log-likelihood pass
