@@ -14,10 +14,10 @@
 //                two-pass radix select over 256-bin histograms, Otsu's threshold), the
 //                flood from the brightest voxel (rows of the box as words in shared memory,
 //                swept until nothing changes; level by level from a queue where the box is wider
-//                than 32, touches an x or y border or exceeds 65536 voxels, the last with one bit
-//                per volume voxel in global memory), each list entry's verdict, and for kept
-//                supervoxels the FP32 centroid in the reference's summation order and the range
-//                of the background-subtracted values.  20,019 supervoxels of 14.5 M voxels:
+//                than 32, touches an x or y border or exceeds 65536 voxels, the last with bits in
+//                global memory, one per volume voxel or list entry), each list entry's verdict, and
+//                for kept supervoxels the FP32 centroid in the reference's summation order and the
+//                range of the background-subtracted values.  20,019 supervoxels of 14.5 M voxels:
 //                1049 us with the queue for all and a warp's centroid over every voxel, 433 us;
 //                bound by each block's chain of barriers, seven blocks an SM (five at 48
 //                registers 490, six 460, eight 433);
@@ -85,7 +85,8 @@ struct FbWork {
   uint32_t* ulin;   // [nvol] lists: linear indices, ascending within a supervoxel
   uint16_t* uval;   // [nvol] their raw values
   uint32_t* queue;  // [nvol] flood queues (a supervoxel's at its list offset)
-  uint32_t* bits;   // [nvol/32] flood: reached voxels (supervoxels whose box exceeds shared memory)
+  uint32_t* bits;   // [nvol/32] flood: reached voxels, in the list form reached list entries (at most
+                    // nvol of them), of supervoxels whose box exceeds shared memory
   uint8_t* ukeep;   // [nvol] 1 where a list entry survived trimming
   int32_t* tcnt;    // [n] voxels kept by trimming
   uint32_t* thr;    // [n] trimming thresholds
@@ -685,6 +686,11 @@ __global__ void __launch_bounds__(kFbTrimThreads, 7) k_fb_trim(const uint32_t* _
     return (y - bx.lo[1]) + bh * (z - bx.lo[2]);
   };
   uint32_t* q = w.queue + a;
+  // The bit of list entry i (voxel v) in w.bits, where the flood leaves shared memory: the
+  // voxel's own where a label volume says whose it is, the entry's where the lists do.  Every
+  // supervoxel then has bits of its own, also where lists hold the same voxel, and queues no
+  // entry twice: its queue has a place for each.
+  auto bit_of = [&](int32_t i, uint32_t v) { return kLists ? (uint32_t)(a + i) : v; };
   if (row_path) {
     const int32_t rows = bh * bd;
     for (int i = t; i < rows; i += kFbTrimThreads) s_cand[i] = s_reach[i] = 0u;
@@ -754,14 +760,17 @@ __global__ void __launch_bounds__(kFbTrimThreads, 7) k_fb_trim(const uint32_t* _
       s_tail = 1;
     }
   } else {
-    // the supervoxel's own voxels' bits (those the flood tests and sets) start clear; a word may
-    // hold another's, whose block does the same
-    for (int32_t i = t; i < N; i += kFbTrimThreads) atomicAnd(&w.bits[lin[i] >> 5], ~(1u << (lin[i] & 31)));
+    // the supervoxel's own bits (those the flood tests and sets) start clear; a word may hold
+    // another's, whose block does the same
+    for (int32_t i = t; i < N; i += kFbTrimThreads) {
+      const uint32_t b = bit_of(i, lin[i]);
+      atomicAnd(&w.bits[b >> 5], ~(1u << (b & 31)));
+    }
     __syncthreads();
     if (t == 0 && val[s_seed] > th) {
-      const uint32_t v = lin[s_seed];
-      atomicOr(&w.bits[v >> 5], 1u << (v & 31));
-      q[0] = v;
+      const uint32_t b = bit_of((int32_t)s_seed, lin[s_seed]);
+      atomicOr(&w.bits[b >> 5], 1u << (b & 31));
+      q[0] = lin[s_seed];
       s_tail = 1;
     }
   }
@@ -798,6 +807,7 @@ __global__ void __launch_bounds__(kFbTrimThreads, 7) k_fb_trim(const uint32_t* _
         for (int j = 0; j < off.n; j++) {
           const int64_t nb = (int64_t)v + off.off[j];
           if (nb < 0 || nb >= nvol) continue;
+          int32_t at = 0;
           if (kLists) {
             // a voxel of this supervoxel (its ascending list, as lower_bound finds it there)
             // brighter than the threshold
@@ -810,11 +820,12 @@ __global__ void __launch_bounds__(kFbTrimThreads, 7) k_fb_trim(const uint32_t* _
                 hi = mid;
             }
             if (lo >= N || (int64_t)lin[lo] != nb || val[lo] <= th) continue;
+            at = lo;
           } else if (label[nb] != want || raw[nb] <= th) {
             continue;
           }
-          const uint32_t bit = 1u << (nb & 31);
-          if (atomicOr(&w.bits[nb >> 5], bit) & bit) continue;
+          const uint32_t b = bit_of(at, (uint32_t)nb), bit = 1u << (b & 31);
+          if (atomicOr(&w.bits[b >> 5], bit) & bit) continue;
           q[atomicAdd(&s_tail, 1u)] = (uint32_t)nb;
         }
       }
@@ -824,7 +835,7 @@ __global__ void __launch_bounds__(kFbTrimThreads, 7) k_fb_trim(const uint32_t* _
   }
   const int32_t kept = (int32_t)s_tail;
   // each list entry's verdict, for the centroid and the emission
-  auto verdict = [&](uint32_t v) -> bool {
+  auto verdict = [&](int32_t i, uint32_t v) -> bool {
     if (row_path) {
       uint32_t bit;
       const int32_t r = row_of(v, &bit);
@@ -837,7 +848,8 @@ __global__ void __launch_bounds__(kFbTrimThreads, 7) k_fb_trim(const uint32_t* _
       return (s_reach[li >> 5] >> (li & 31)) & 1u;
     }
     // the flood's bits were set by atomics at L2: read them there
-    return (__ldcg(&w.bits[v >> 5]) >> (v & 31)) & 1u;
+    const uint32_t b = bit_of(i, v);
+    return (__ldcg(&w.bits[b >> 5]) >> (b & 31)) & 1u;
   };
   if (t == 0) w.tcnt[s] = kept;
   if (kept < min_size) {  // erased: its verdicts are not read
@@ -859,7 +871,7 @@ __global__ void __launch_bounds__(kFbTrimThreads, 7) k_fb_trim(const uint32_t* _
     if (i < N) {
       v = lin[i];
       r = val[i];
-      in = verdict(v);
+      in = verdict(i, v);
       keep[i] = in ? 1 : 0;
     }
     const unsigned m = __ballot_sync(0xffffffffu, in);
