@@ -168,6 +168,7 @@ __device__ __forceinline__ FrameDesc load_desc(const DevPlan& P, int f) { return
 }  // namespace
 
 
+constexpr int kMaxGridDim = 1024;  // cells along an axis
 // Grid geometry over the bounding box [lo, hi] (scaled space): cubic cells of side h,
 // about one reference per cell, at most budget-1 cells in total.
 __device__ void set_geometry(FrameState* S, const float* lo, const float* hi, int n_ref, int cell_budget,
@@ -187,7 +188,7 @@ __device__ void set_geometry(FrameState* S, const float* lo, const float* hi, in
   for (int guard = 0; guard < 400; guard++) {
     long long tot = 1;
     for (int d = 0; d < 3; d++) {
-      dims[d] = max(1, min(1024, (int)ceilf(ext[d] / h)));
+      dims[d] = max(1, min(kMaxGridDim, (int)ceilf(ext[d] / h)));
       tot *= dims[d];
     }
     if (tot <= budget) break;
@@ -3071,12 +3072,15 @@ void launch_export(const DevPlan& P, cudaStream_t st) { k_export<<<P.max_gchunks
 // 4 * budget bytes start at zero).
 struct SaScratch {
   FrameState* S;   // the grid geometry (lo, h, inv_h, dims, n_cells)
-  unsigned* box;   // keys of the box (see box_key), arrived blocks, next free place
+  unsigned* box;   // keys of the box (see box_key), arrived blocks, next free place, and from
+                   // kSaExtent on the extent of the cells that hold references (see k_sa_count)
   int* cnt;        // [budget] references per cell
   int* start;      // [budget] the cell's first place
   int2* place;     // [nref] cell (-1: in none) and place within it
   float4* refs;    // [nref] coordinates and index, cell by cell
 };
+constexpr int kSaExtent = 8;
+static_assert((kSaExtent + 6) * 4 <= (int)(kSaClear - kSaBox), "the header holds the box and the extent");
 static_assert(sizeof(FrameState) <= kSaBox, "the grid geometry record fits its part of the scratch header");
 
 static SaScratch sa_carve(char* buf, int32_t nref) {
@@ -3155,21 +3159,40 @@ __global__ void __launch_bounds__(256) k_sa_bounds(const float* __restrict__ q, 
 // comp 1) or SoA x-block, y-block, z-block (step 1, comp nref).
 __global__ void __launch_bounds__(256) k_sa_count(const float* __restrict__ ref, int nref, int step, int64_t comp,
                                                   float s0, float s1, float s2, SaScratch w) {
+  // the block's extent of cells, as maxima over cleared words: kMaxGridDim - the smallest, and one
+  // more than the largest
+  __shared__ unsigned ext[6];
+  if (threadIdx.x < 6) ext[threadIdx.x] = 0;
+  __syncthreads();
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= nref) return;
-  const float* rk = ref + (int64_t)k * step;
-  const float ys[3] = {rk[0] * s0, rk[comp] * s1, rk[2 * comp] * s2};
-  int2 p = make_int2(0, 0);
-  for (int d = 0; d < 3; d++)
-    if (!isfinite(ys[d]) || fabsf(ys[d]) >= 1e25f) p.x = -1;
-  if (p.x == 0) {
-    const int cx = cell_coord(ys[0], w.S->lo[0], w.S->inv_h, w.S->dims[0]);
-    const int cy = cell_coord(ys[1], w.S->lo[1], w.S->inv_h, w.S->dims[1]);
-    const int cz = cell_coord(ys[2], w.S->lo[2], w.S->inv_h, w.S->dims[2]);
-    p.x = (cz * w.S->dims[1] + cy) * w.S->dims[0] + cx;
-    p.y = atomicAdd(&w.cnt[p.x], 1);
+  int2 p = make_int2(-1, 0);
+  unsigned m[6] = {0, 0, 0, 0, 0, 0};
+  if (k < nref) {
+    const float* rk = ref + (int64_t)k * step;
+    const float ys[3] = {rk[0] * s0, rk[comp] * s1, rk[2 * comp] * s2};
+    bool in = true;
+    for (int d = 0; d < 3; d++)
+      if (!isfinite(ys[d]) || fabsf(ys[d]) >= 1e25f) in = false;
+    if (in) {
+      int c[3];
+#pragma unroll
+      for (int d = 0; d < 3; d++) {
+        c[d] = cell_coord(ys[d], w.S->lo[d], w.S->inv_h, w.S->dims[d]);
+        m[d] = (unsigned)(kMaxGridDim - c[d]);
+        m[3 + d] = (unsigned)(c[d] + 1);
+      }
+      p.x = (c[2] * w.S->dims[1] + c[1]) * w.S->dims[0] + c[0];
+      p.y = atomicAdd(&w.cnt[p.x], 1);
+    }
+    w.place[k] = p;
   }
-  w.place[k] = p;
+#pragma unroll
+  for (int d = 0; d < 6; d++) {
+    m[d] = __reduce_max_sync(0xffffffffu, m[d]);
+    if ((threadIdx.x & 31) == 0 && m[d]) atomicMax(&ext[d], m[d]);
+  }
+  __syncthreads();
+  if (threadIdx.x < 6 && ext[threadIdx.x]) atomicMax(&w.box[kSaExtent + threadIdx.x], ext[threadIdx.x]);
 }
 
 // A warp per x-row of cells: the row's references get one contiguous range, its cells in
@@ -3212,77 +3235,187 @@ __global__ void __launch_bounds__(256) k_sa_fill(const float* __restrict__ ref, 
 template <typename F>
 __device__ __forceinline__ void sa_scan_cell(const SaScratch& w, int cell, float q0, float q1, float q2, const float* s,
                                              F take) {
-  const int b = w.start[cell], e = b + w.cnt[cell];
+  const int n = w.cnt[cell];
+  if (n == 0) return;  // (most cells of a far query's rings)
+  const int b = w.start[cell], e = b + n;
   for (int k = b; k < e; ++k) {
     const float4 rr = w.refs[k];
     take(knn_dist(q0, q1, q2, rr.x, rr.y, rr.z, s), __float_as_int(rr.w));
   }
 }
 
-// The N nearest of one query by one thread: rings of cells at growing Chebyshev distance
-// around the query's cell, passing over cells farther than the N-th distance so far.  Ends
-// when the N-th distance is strictly below the bound of every cell not visited.
+// The rings of cells of a ring search: those at Chebyshev distance first .. last from the query's
+// cell, clipped to the cells [lo, hi] that hold the references.  A query far from all of them
+// starts at their box: no ring before it holds a cell.  first > last without a reference.
+struct SaRings {
+  int lo[3], hi[3], first, last;
+  __device__ __forceinline__ SaRings(const GridPlace& p, const SaScratch& w) {
+    first = last = 0;
+    const unsigned* e = w.box + kSaExtent;
+    if (e[3] == 0) first = 1;  // no reference in the grid
+#pragma unroll
+    for (int a = 0; a < 3; a++) {
+      lo[a] = kMaxGridDim - (int)e[a];
+      hi[a] = (int)e[3 + a] - 1;
+      first = max(first, max(lo[a] - p.c[a], p.c[a] - hi[a]));
+      last = max(last, max(p.c[a] - lo[a], hi[a] - p.c[a]));
+    }
+    if (e[3] == 0) last = 0;
+  }
+  // A squared distance below which every reference lies in the rings up to r (infinite when there
+  // is no other): the nearest side behind which rings are left.  A query past the grid's edge (or
+  // on a face along an axis of few cells) is not held back by the sides that have none.
+  __device__ __forceinline__ float bound2(const GridPlace& p, int r, float h) const {
+    float lb = kInfF;
+#pragma unroll
+    for (int a = 0; a < 3; a++) {
+      if (p.c[a] - r > lo[a]) lb = fminf(lb, p.f0[a] + r * h);
+      if (p.c[a] + r < hi[a]) lb = fminf(lb, p.f1[a] + r * h);
+    }
+    if (lb == kInfF) return kInfF;
+    const float m = lb - (p.eps0 + 1e-6f * lb);
+    return m > 0.0f ? m * m : 0.0f;
+  }
+};
+
+// The N nearest of one query by one thread: the cells of one ring after the other, passing over
+// those farther than the N-th distance so far.  Ends when the N-th distance is strictly below the
+// bound of every cell not visited.  A ring's cells are taken face by face -- across z, across y,
+// across x -- so that none off the ring is looked at.  The list is a local of the function: by
+// reference it would lie in memory, and a query far from a crowd of references compares with it
+// thousands of times.
 template <int N>
 __device__ __noinline__ void sa_search_thread(float q0, float q1, float q2, const float* s, const GridGeom& g,
-                                              const SaScratch& w, TopN<N>& best) {
+                                              const SaScratch& w, TopN<N>& out) {
   const GridPlace p(q0, q1, q2, s, g);
+  TopN<N> best;
   topn_init<N>(best);
-  const int maxr = max(g.dims[0], max(g.dims[1], g.dims[2]));
-  for (int r = 0; r <= maxr; ++r) {
-    const int z0 = max(p.c[2] - r, 0), z1 = min(p.c[2] + r, g.dims[2] - 1);
-    const int y0 = max(p.c[1] - r, 0), y1 = min(p.c[1] + r, g.dims[1] - 1);
-    for (int z = z0; z <= z1; ++z) {
+  const SaRings R(p, w);
+  // the cells [x0, x1] x [y0, y1] x [z0, z1]
+  auto scan = [&](int x0, int x1, int y0, int y1, int z0, int z1) {
+    for (int z = z0; z <= z1; z++) {
       const float gz = p.gap2(2, z - p.c[2], g.h);
       if (gz > best.d[N - 1]) continue;
-      const bool zedge = (z == p.c[2] - r) || (z == p.c[2] + r);
-      for (int yy = y0; yy <= y1; ++yy) {
-        const float gy = gz + p.gap2(1, yy - p.c[1], g.h);
+      for (int y = y0; y <= y1; y++) {
+        const float gy = gz + p.gap2(1, y - p.c[1], g.h);
         if (gy > best.d[N - 1]) continue;
-        const bool edge = zedge || (yy == p.c[1] - r) || (yy == p.c[1] + r);
-        const int row = (z * g.dims[1] + yy) * g.dims[0];
-        const int step = edge || r == 0 ? 1 : 2 * r;
-        for (int x = p.c[0] - r; x <= p.c[0] + r; x += step) {
-          if (x < 0 || x >= g.dims[0] || gy + p.gap2(0, x - p.c[0], g.h) > best.d[N - 1]) continue;
+        const int row = (z * g.dims[1] + y) * g.dims[0];
+        // (a row's cells lie one after the other in w.refs: one that holds nothing is passed over)
+        if (x0 < x1 && w.start[row + x1] + w.cnt[row + x1] == w.start[row + x0]) continue;
+        for (int x = x0; x <= x1; x++) {
+          if (gy + p.gap2(0, x - p.c[0], g.h) > best.d[N - 1]) continue;
           sa_scan_cell(w, row + x, q0, q1, q2, s, [&](float d, int id) { topn_insert<N>(best, d, id); });
         }
       }
     }
-    if (best.d[N - 1] < p.bound2(r, g.h)) break;
+  };
+  for (int r = R.first; r <= R.last; ++r) {
+    int lo[3], hi[3], in0[3], in1[3];
+#pragma unroll
+    for (int a = 0; a < 3; a++) {
+      lo[a] = max(p.c[a] - r, R.lo[a]);
+      hi[a] = min(p.c[a] + r, R.hi[a]);
+      in0[a] = max(p.c[a] - r + 1, R.lo[a]);
+      in1[a] = min(p.c[a] + r - 1, R.hi[a]);
+    }
+    for (int side = r == 0 ? 1 : 0; side < 2; side++) {  // (r = 0: the query's cell, once)
+      const int d = side ? r : -r, x = p.c[0] + d, y = p.c[1] + d, z = p.c[2] + d;
+      if (z >= R.lo[2] && z <= R.hi[2]) scan(lo[0], hi[0], lo[1], hi[1], z, z);
+      if (y >= R.lo[1] && y <= R.hi[1]) scan(lo[0], hi[0], y, y, in0[2], in1[2]);
+      if (x >= R.lo[0] && x <= R.hi[0]) scan(x, x, in0[1], in1[1], in0[2], in1[2]);
+    }
+    if (best.d[N - 1] < R.bound2(p, r, g.h)) break;
   }
+  out = best;
 }
 
-// The same by the G lanes of a group, a ring at a time from the 27 cells around the query:
-// the lanes split a ring's cells and merge their lists after it.
+// The same by the G lanes of a group.  A ring's cells are stretches of x-rows, each one range of
+// w.refs: whole rows on the faces across z and y, single cells on those across x.  A lane takes
+// a stretch's range, then the group scans the ranges that hold anything, a reference a lane, and
+// merges its lists when something was kept.  Rings 0 and 1 are one.  20,000 queries over a box,
+// 20,000 references in one corner of it, K = 10: 3.0 ms (a thread per query over rings clipped to
+// the grid alone 52); half of the box 0.34 ms (1.6); eight spots of one slice 1.2 ms (13); one end
+// of a line 0.13 ms (3.1).
 template <int G, int N>
 __device__ __noinline__ void sa_search_group(float q0, float q1, float q2, const float* s, const GridGeom& g,
                                              const SaScratch& w, TopN<N>& best, int gl, unsigned gmask) {
   const GridPlace p(q0, q1, q2, s, g);
   topn_init<N>(best);
-  const int maxr = max(1, max(g.dims[0], max(g.dims[1], g.dims[2])));
-  for (int r = 1; r <= maxr; ++r) {
+  const SaRings R(p, w);
+  for (int r = R.first == 0 ? 1 : R.first; r <= max(R.last, R.first == 0 ? 1 : 0); ++r) {
     TopN<N> t;
     topn_init<N>(t);
+    bool kept = false;
     const float td = best.d[N - 1];
     const int ti = best.i[N - 1];
-    const int side = 2 * r + 1, cube = side * side * side;
-    for (int idx = gl; idx < cube; idx += G) {
-      const int dx = idx % side - r, dy = (idx / side) % side - r, dz = idx / (side * side) - r;
-      if (r > 1 && max(abs(dx), max(abs(dy), abs(dz))) != r) continue;
-      if (p.gap2(0, dx, g.h) + p.gap2(1, dy, g.h) + p.gap2(2, dz, g.h) > td) continue;
-      const int x = p.c[0] + dx, yy = p.c[1] + dy, z = p.c[2] + dz;
-      if (x < 0 || yy < 0 || z < 0 || x >= g.dims[0] || yy >= g.dims[1] || z >= g.dims[2]) continue;
-      sa_scan_cell(w, (z * g.dims[1] + yy) * g.dims[0] + x, q0, q1, q2, s, [&](float d, int id) {
-        if (!before(td, ti, d, id)) topn_insert<N>(t, d, id);
-      });
-    }
-    if (gl == 0) {
+    // the ring's extent clipped to the references' cells, and without its faces
+    int lo[3], hi[3], in0[3], n_in[3];
+    bool face0[3], face1[3];
 #pragma unroll
-      for (int j = 0; j < N; j++) topn_insert<N>(t, best.d[j], best.i[j]);
+    for (int a = 0; a < 3; a++) {
+      const int c0 = p.c[a] - r, c1 = p.c[a] + r;
+      face0[a] = c0 >= R.lo[a] && c0 <= R.hi[a];
+      face1[a] = c1 >= R.lo[a] && c1 <= R.hi[a];
+      lo[a] = max(c0, R.lo[a]);
+      hi[a] = min(c1, R.hi[a]);
+      in0[a] = max(c0 + 1, R.lo[a]);
+      n_in[a] = max(min(c1 - 1, R.hi[a]) - in0[a] + 1, 0);
     }
-    TopN<N> merged;
-    group_merge_topn<G, N>(t, merged, gmask);
-    best = merged;
-    if (best.d[N - 1] < p.bound2(r, g.h)) break;
+    const bool whole = r == 1 && R.first == 0;
+    const int ny = hi[1] - lo[1] + 1, area = n_in[1] * n_in[2];
+    // stretches: the rows across z, the rows across y, the cells across x (whole: every row)
+    const int z_rows = whole ? ny * (hi[2] - lo[2] + 1) : (face0[2] + face1[2]) * ny;
+    const int y_rows = whole ? 0 : (face0[1] + face1[1]) * n_in[2];
+    const int total = z_rows + y_rows + (whole ? 0 : (face0[0] + face1[0]) * area);
+    for (int i0 = 0; i0 < total; i0 += G) {
+      int i = i0 + gl, b = 0, e = 0;
+      if (i < total) {
+        int y, z, xa = lo[0], xb = hi[0];
+        if (i < z_rows) {
+          y = lo[1] + i % ny;
+          z = whole ? lo[2] + i / ny : face0[2] && i < ny ? p.c[2] - r : p.c[2] + r;
+        } else if ((i -= z_rows) < y_rows) {
+          z = in0[2] + i % n_in[2];
+          y = face0[1] && i < n_in[2] ? p.c[1] - r : p.c[1] + r;
+        } else {
+          i -= y_rows;
+          xa = xb = face0[0] && i < area ? p.c[0] - r : p.c[0] + r;
+          if (i >= area) i -= area;
+          y = in0[1] + i % n_in[1];
+          z = in0[2] + i / n_in[1];
+        }
+        const float gap = p.gap2(1, y - p.c[1], g.h) + p.gap2(2, z - p.c[2], g.h) +
+                          (xa == xb ? p.gap2(0, xa - p.c[0], g.h) : 0.0f);
+        if (!(gap > td)) {
+          const int row = (z * g.dims[1] + y) * g.dims[0];
+          b = w.start[row + xa];
+          e = w.start[row + xb] + w.cnt[row + xb];
+        }
+      }
+      for (unsigned m = __ballot_sync(gmask, e > b) & gmask; m; m &= m - 1) {
+        const int from = __ffs(m) - 1, eb = __shfl_sync(gmask, e, from);
+        for (int k = __shfl_sync(gmask, b, from) + gl; k < eb; k += G) {
+          const float4 rr = w.refs[k];
+          const float d = knn_dist(q0, q1, q2, rr.x, rr.y, rr.z, s);
+          const int id = __float_as_int(rr.w);
+          if (!before(td, ti, d, id)) {
+            topn_insert<N>(t, d, id);
+            kept = true;
+          }
+        }
+        __syncwarp(gmask);
+      }
+    }
+    if (__any_sync(gmask, kept)) {
+      if (gl == 0) {
+#pragma unroll
+        for (int j = 0; j < N; j++) topn_insert<N>(t, best.d[j], best.i[j]);
+      }
+      TopN<N> merged;
+      group_merge_topn<G, N>(t, merged, gmask);
+      best = merged;
+    }
+    if (best.d[N - 1] < R.bound2(p, r, g.h)) break;
   }
 }
 
@@ -3320,6 +3453,12 @@ __device__ __forceinline__ float sa_next_radius(float rad, int n) {
   const float f = cbrtf((n < K ? 2.0f * K : 1.5f * K) / ((float)n + 0.5f));
   return rad * (n < K ? fminf(fmaxf(f, 1.25f), 2.0f) : fminf(f, 0.9f));
 }
+
+// Blocks an SM of the two query kernels: what the collecting search needs, so that the ring search
+// they fall back to, which keeps more in registers, does not cost the others theirs (1.43 M voxels,
+// K = 5: 173 us with eight blocks, 178 with the seven of 72 registers).
+constexpr int sa_warp_blocks(int K) { return K <= 4 ? 9 : K <= 6 ? 8 : K == 7 ? 7 : K <= 9 ? 6 : 5; }
+constexpr int sa_group_blocks(int K) { return K <= 2 ? 10 : K == 3 ? 9 : K <= 5 ? 8 : K == 6 ? 7 : K == 7 ? 6 : K <= 9 ? 5 : 4; }
 
 constexpr int kSaKeep = 64;       // references kept per query of a group
 constexpr int kSaKeepWarp = 128;  // references kept per warp of queries
@@ -3436,7 +3575,7 @@ __device__ __forceinline__ bool sa_select(const float* qv, const float* s, const
 // distances too close to tell apart by their keys) runs the ring search.  1.43 M voxels against
 // 2000 references: 133 us, 71% of the issue slots busy (a thread per query: 239 us).
 template <int K, bool kMark>
-__global__ void __launch_bounds__(128) k_sa_query_warp(const float* __restrict__ q, int64_t nq,
+__global__ void __launch_bounds__(128, sa_warp_blocks(K)) k_sa_query_warp(const float* __restrict__ q, int64_t nq,
                                                        const float* __restrict__ ref, int nref, int step,
                                                        int64_t comp, float s0, float s1, float s2, SaScratch w,
                                                        int32_t* ind, float* dist) {
@@ -3498,7 +3637,8 @@ __global__ void __launch_bounds__(128) k_sa_query_warp(const float* __restrict__
     waits = waits && !mine;
   }
   if (!done) {
-    sa_search_thread<K>(qv[0], qv[1], qv[2], sc, g, w, t);
+    topn_init<K>(t);
+    if (fin) sa_search_thread<K>(qv[0], qv[1], qv[2], sc, g, w, t);
     if (!(t.d[K - 1] < kInfF)) {  // fewer than K finite distances: every reference point
       topn_init<K>(t);
       for (int k = 0; k < nref; k++) {
@@ -3519,7 +3659,7 @@ __global__ void __launch_bounds__(128) k_sa_query_warp(const float* __restrict__
 // 20,007 references, K = 10: 48 us, bound by the chain of dependent loads (a thread per query,
 // 625 warps on the device: 195 us).
 template <int G, int K, bool kMark>
-__global__ void __launch_bounds__(128) k_sa_query_group(const float* __restrict__ q, int64_t nq,
+__global__ void __launch_bounds__(128, sa_group_blocks(K)) k_sa_query_group(const float* __restrict__ q, int64_t nq,
                                                         const float* __restrict__ ref, int nref, int step,
                                                         int64_t comp, float s0, float s1, float s2, SaScratch w,
                                                         int32_t* ind, float* dist) {
@@ -3533,7 +3673,8 @@ __global__ void __launch_bounds__(128) k_sa_query_group(const float* __restrict_
   const float qv[3] = {q[i], q[nq + i], q[2 * nq + i]};
   const float yq[3] = {qv[0] * s0, qv[1] * s1, qv[2] * s2};
   const GridGeom g = sa_geometry(w);
-  if (isfinite(yq[0]) && isfinite(yq[1]) && isfinite(yq[2])) {
+  const bool fin = isfinite(yq[0]) && isfinite(yq[1]) && isfinite(yq[2]);
+  if (fin) {
     const float eps0 = 4e-3f + 1e-6f * fmaxf(fmaxf(fabsf(yq[0]), fabsf(yq[1])), fabsf(yq[2]));
     float rad = sa_first_radius<K>(g.h);
     for (int u = 0; u < kSaTries; u++) {
@@ -3553,11 +3694,14 @@ __global__ void __launch_bounds__(128) k_sa_query_group(const float* __restrict_
         }
         return;
       }
+      if (n == 0) break;  // far from the references: the ring search starts at them
       rad = sa_next_radius<K>(rad, n);
     }
   }
   TopN<K> t;
-  sa_search_group<G, K>(qv[0], qv[1], qv[2], sc, g, w, t, gl, gmask);
+  topn_init<K>(t);
+  // (no distance of a query with a NaN or infinite coordinate is finite)
+  if (fin) sa_search_group<G, K>(qv[0], qv[1], qv[2], sc, g, w, t, gl, gmask);
   if (!(t.d[K - 1] < kInfF)) {
     TopN<K> mine;
     topn_init<K>(mine);
