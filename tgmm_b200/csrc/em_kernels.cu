@@ -1579,7 +1579,6 @@ __global__ void __launch_bounds__(kGChunk) k_kill_prep(DevPlan P) {
 // convergence test for that frame.
 // ===========================================================================
 constexpr float kL2E = 1.4426950408889634f;  // log2(e)
-constexpr double kFracScale = 1099511627776.0;  // 2^40
 
 __device__ __forceinline__ float ex2_approx(float x) {
   float y;
@@ -1927,17 +1926,11 @@ __device__ __forceinline__ void ll_consume(const VoxelEval64& eval, const float*
   }
 }
 
-// Order-free accumulation: a double becomes an (integer, 2^-40 fraction) pair, and pairs
-// add as integers, so a total does not depend on the order of its parts.
-__device__ __forceinline__ void fixed_acc(long long& ip, unsigned long long& fp, double v) {
-  const double fl = floor(v);
-  ip += (long long)fl;
-  fp += (unsigned long long)((v - fl) * kFracScale);
-}
-
+// A frame's order-free sum (see fixed_acc); its fractions come carried from each warp.
 __device__ __forceinline__ double fixed_read(const long long* ip, const unsigned long long* fp) {
-  const long long i = *(volatile const long long*)ip;
-  const unsigned long long f = *(volatile const unsigned long long*)fp;
+  long long i = *(volatile const long long*)ip;
+  unsigned long long f = *(volatile const unsigned long long*)fp;
+  fixed_carry(i, f);
   return (double)i + (double)f / kFracScale;
 }
 
@@ -2003,6 +1996,8 @@ __global__ void __launch_bounds__(kLLWarps * 32, kLLBlocks) k_ll_pass(DevPlan P)
   auto publish = [&]() {
     if (lane == 0 && acc_n > 0) {
       FrameState* Sp = &P.state[acc_f];
+      fixed_carry(acc_i0, acc_r0);
+      fixed_carry(acc_i1, acc_r1);
       atomicAdd((unsigned long long*)&Sp->ll_int[0], (unsigned long long)acc_i0);
       atomicAdd((unsigned long long*)&Sp->ll_int[1], (unsigned long long)acc_i1);
       atomicAdd(&Sp->ll_frac[0], acc_r0);
@@ -2548,8 +2543,11 @@ __global__ void __launch_bounds__(kLSWarps * 32, kLSBlocks) k_ll_stream(DevPlan 
   Sh.dr[lane] = 0;
   auto publish = [&]() {
     if (acc_n > 0) {
+      // (what the kept window leaves out was subtracted: ri, rr is a sum of the kept parts alone)
       long long ri = ai + Sh.di[lane];
       unsigned long long rr = ar + Sh.dr[lane];
+      fixed_carry(ai, ar);
+      fixed_carry(ri, rr);
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) {
         ai += __shfl_xor_sync(0xffffffffu, ai, o);
@@ -2559,6 +2557,8 @@ __global__ void __launch_bounds__(kLSWarps * 32, kLSBlocks) k_ll_stream(DevPlan 
       }
       if (lane == 0) {
         FrameState* S = &P.state[acc_f];
+        fixed_carry(ai, ar);
+        fixed_carry(ri, rr);
         atomicAdd((unsigned long long*)&S->ll_int[0], (unsigned long long)ai);
         atomicAdd((unsigned long long*)&S->ll_int[1], (unsigned long long)ri);
         atomicAdd(&S->ll_frac[0], ar);

@@ -31,6 +31,22 @@ constexpr double kLn2 = 0.69314718055994530942;
 constexpr double kPi = 3.14159265358979323846;
 constexpr double kLnTwoPi = 1.83787706640934548356;  // ln(2*pi)
 
+// Order-free accumulation: a double becomes an (integer, 2^-40 fraction) pair, and pairs add as
+// integers, so a total does not depend on the order of its parts.  A fraction word holds 2^24
+// parts; fixed_carry moves its whole units into the integer and leaves less than one.  Each lane
+// carries before it adds to others' words, so that the limit is 2^24 parts a lane between two
+// publications, and 2^24 publications a frame (at most one a warp of the pass).
+constexpr double kFracScale = 1099511627776.0;  // 2^40
+TG_HD void fixed_acc(long long& ip, unsigned long long& fp, double v) {
+  const double fl = floor(v);
+  ip += (long long)fl;
+  fp += (unsigned long long)((v - fl) * kFracScale);
+}
+TG_HD void fixed_carry(long long& ip, unsigned long long& fp) {
+  ip += (long long)(fp >> 40);
+  fp &= (1ull << 40) - 1;
+}
+
 TG_HD bool is_dead_prior(double m_o0) { return m_o0 < -1e31; }
 
 // psi(x) for x > 0: Bernardo's AS 103 as modified by Minka -- a small-argument
