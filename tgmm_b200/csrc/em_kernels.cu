@@ -393,7 +393,7 @@ __device__ __forceinline__ double write_records(const DevPlan& P, const FrameDes
   L[3] = -0.5 * nu * W[3];
   L[4] = -nu * W[4];
   L[5] = -0.5 * nu * W[5];
-  L[6] = 0.5 * log(det3(W) * nu * nu * nu * (alpha * alpha)) - 1.5 * kLnTwoPi;
+  L[6] = log_weight(det3(W) * nu * nu * nu, alpha);
   L[7] = m[0];
   L[8] = m[1];
   L[9] = m[2];

@@ -328,6 +328,15 @@ TG_HD void regularize_W(double* Wk, double nu, const RegConst& rc) {
   for (int e = 0; e < 6; e++) Wk[e] = W[e] * (double)(rc.scale[ia[e]] * rc.scale[ib[e]]);
 }
 
+// ln of a component's weight without the frame's alpha total: ln(alpha) + ln(p)/2 - 3 ln(2 pi)/2 for
+// p = det(nu W).  One logarithm where the product under it is a normal number; an alpha that is
+// not positive has none (NaN, or -inf at 0), and one whose square would underflow keeps its own.
+TG_HD double log_weight(double p, double alpha) {
+  const double x = p * (alpha * alpha);
+  if (alpha > 1e-100 && x > 1e-290 && x < 1e290) return 0.5 * log(x) - 1.5 * kLnTwoPi;
+  return 0.5 * log(p) - 1.5 * kLnTwoPi + log(alpha);
+}
+
 // E[ln |Lambda|] = 3 ln 2 + ln det W + sum_{i=0..2} psi((nu + 1 - i)/2)
 // (GMEMupdateCUDA.cu:553-576; the index starts at 0 as in the reference).
 TG_HD double expected_log_det(const double* W, double nu) {
