@@ -304,10 +304,10 @@ TG_HD void regularize_W(double* Wk, double nu, const RegConst& rc) {
   const int pa[3] = {0, 0, 1}, pb[3] = {1, 2, 2};
   for (int q = 0; q < 3; q++) {
 #if TG_RCP
-    // the clamp above left them positive
-    if (d[pa[q]] > rc.max_exc * d[pb[q]])
+    // the clamp above left them with one sign, nu's
+    if (fabs(d[pa[q]]) > rc.max_exc * fabs(d[pb[q]]))
       d[pa[q]] = rc.max_exc * d[pb[q]];
-    else if (d[pb[q]] > rc.max_exc * d[pa[q]])
+    else if (fabs(d[pb[q]]) > rc.max_exc * fabs(d[pa[q]]))
       d[pb[q]] = rc.max_exc * d[pa[q]];
 #else
     const double r = d[pa[q]] / d[pb[q]];
