@@ -3804,25 +3804,42 @@ cudaError_t knn_grid_in_scratch(const float* q, int64_t nq, const float* ref, in
 // GaussianMixtureModel.cpp:892-910; N_k = nu_k - nu_o as copyFromGMEM_CUDA/updateNk
 // derive it; then nu_k *= 2, W_k /= 2 as mainTrackingGaussianMixtureModel.cpp:961-969).
 // kPriorsPerBlock records a block.  The optional alpha total (alpha_k is not written here) is
-// the same fixed-order sum in every block, so no block waits for another: 8 bytes of each
-// record read again per block, against a second launch and a place for the total.  Bound by
-// latency; 5000 records: 76 us in one block, 9.4 us this way.
+// the same fixed-order sum in every block, so no block waits for another: a 32-byte sector of
+// each record read again per block, against a second launch.  Bound by latency; 5000 records: 76
+// us in one block, 9.4 us this way.  Those reads grow with the square of the record count: from
+// kPriorsOwnTotal records on one block forms the total and writes alpha_o ahead of the others.
 // ---------------------------------------------------------------------------
 constexpr int kPriorsPerBlock = 256;
+// Every block the total / one block ahead: 20,000 records 28 / 41 us, 40,000 63 / 64, 60,000 85 /
+// 87, 100,000 181 / 132, 1 M 13,893 / 1204 (all in one block 14,801).
+constexpr int kPriorsOwnTotal = 65536;
+
+// The alpha total of a block of 1024 threads: thread-strided sums in index order, a warp's lanes,
+// then the warps.
+__device__ __forceinline__ double priors_alpha_total(const TgmmGaussian* gm, int n, double* sh) {
+  double a = 0.0;
+#pragma unroll 8
+  for (int k = threadIdx.x; k < n; k += 1024) a += gm[k].alpha_k;
+  a = warp_sum(a);
+  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = a;
+  __syncthreads();
+  double total = 0.0;
+#pragma unroll
+  for (int i = 0; i < 32; i++) total += sh[i];
+  return total;
+}
+
+__global__ void __launch_bounds__(1024) k_priors_alpha(TgmmGaussian* gm, int n, double ap) {
+  __shared__ double sh[32];
+  const double total = priors_alpha_total(gm, n, sh);
+  if (total >= 0.0)
+    for (int k = threadIdx.x; k < n; k += 1024) gm[k].alpha_o = total * TGMM_MIN_PI_FOR_DEAD * ap;
+}
+
 __global__ void __launch_bounds__(1024) k_update_priors(TgmmGaussian* gm, int n, double bp, double np, double ap,
                                                         double atot, int compute) {
   __shared__ double sh[32];
-  if (compute && atot < 0.0) {
-    double a = 0.0;
-#pragma unroll 8
-    for (int k = threadIdx.x; k < n; k += 1024) a += gm[k].alpha_k;
-    a = warp_sum(a);
-    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = a;
-    __syncthreads();
-    atot = 0.0;
-#pragma unroll
-    for (int i = 0; i < 32; i++) atot += sh[i];
-  }
+  if (compute && atot < 0.0) atot = priors_alpha_total(gm, n, sh);
   const int k = blockIdx.x * kPriorsPerBlock + threadIdx.x;
   if (threadIdx.x >= kPriorsPerBlock || k >= n) return;
   TgmmGaussian& g = gm[k];
@@ -3846,6 +3863,10 @@ __global__ void __launch_bounds__(1024) k_update_priors(TgmmGaussian* gm, int n,
 
 cudaError_t update_priors_device(TgmmGaussian* gm, int32_t n, double bp, double np, double ap, double atot,
                                  int compute, cudaStream_t st) {
+  if (compute && atot < 0.0 && n >= kPriorsOwnTotal) {
+    k_priors_alpha<<<1, 1024, 0, st>>>(gm, n, ap);
+    compute = 0;
+  }
   k_update_priors<<<(n + kPriorsPerBlock - 1) / kPriorsPerBlock, 1024, 0, st>>>(gm, n, bp, np, ap, atot, compute);
   return cudaGetLastError();
 }
