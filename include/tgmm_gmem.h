@@ -150,7 +150,10 @@ typedef struct TgmmEmStats {
   int32_t device_flags;     /* bit mask of device-side anomaly flags (0 = none) */
   int32_t knn_searches;     /* supervoxel kNN grid searches after the first iteration: the
                                later iterations take each supervoxel's five candidates from
-                               its list of 8 nearest unless its Gaussians moved too far */
+                               its list of 8 nearest unless its Gaussians moved too far.  A
+                               count of work, not a result: it depends on the path taken (a
+                               search in the kNN/E-step's own kernel may keep fewer than 8,
+                               and then searches again earlier than one in the voxel pass) */
   int32_t reserved;
 } TgmmEmStats;
 

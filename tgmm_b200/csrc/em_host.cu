@@ -106,7 +106,10 @@ int report_error(int code, const char* what, cudaError_t e) { return fail(code, 
 // 0.2 ms the small calls run for.  Requests up to kScratchSmall come from a pool of this
 // library's own on each device, which keeps up to kScratchKept of unused memory (and hands back
 // the rest as the default pool does) until the process ends; larger ones from the default pool,
-// as does a stream being captured, whose allocations belong to the graph.
+// as does a stream being captured, whose allocations belong to the graph.  The line keeps what the
+// library holds back out of sight small: a program that watches or limits its device memory
+// through the default pool still finds every larger request there (the kNN from 26,197 references
+// on, at 40 bytes each), at that pool's cost.
 constexpr size_t kScratchSmall = (size_t)1 << 20;
 constexpr uint64_t kScratchKept = (uint64_t)64 << 20;  // two of the pool's 32-MiB pieces
 constexpr int kScratchDevices = 64;

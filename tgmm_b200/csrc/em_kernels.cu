@@ -234,7 +234,7 @@ __device__ void write_sv_rec(const DevPlan& P, const FrameDesc& D, int f, int s,
   SvLL l;
   l.v0 = D.vox_base + (nt ? a : 0);
   l.nv = nv;
-  l.ntiles = nt;
+  l.pad = 0;
   l.frame = f;
   l.frame_nsv = D.n_sv;
   l.c0 = r.c0;
@@ -583,10 +583,13 @@ __global__ void __launch_bounds__(256) k_order_scatter(DevPlan P) {
 // knn_estep: a group of G lanes per supervoxel (32 / G supervoxels per warp; G = 4, 8, 16
 // or 32, chosen per plan, by tgmm_plan_autotune or tgmm_plan_set_knn_group; every G gives
 // the same bits).
-// Exact 5-NN of the centroid among the frame's Gaussian centres: the group's lanes split
-// each ring of grid cells, keep private top-5 lists pruned by the group's current fifth
-// distance, and after each ring the lists are merged by five rounds of a group-wide
-// (distance, index) arg-min.  Then the E-step from the supervoxel's moments, candidate j
+// Exact 5-NN of the centroid among the frame's Gaussian centres: from the supervoxel's list of
+// kNbr near Gaussians while that settles them, else by a search of the grid that also renews the
+// list.  The kernel of its own collects and ranks the references within a limit
+// (knn_group_collect); where that does not settle it, and inside the voxel pass, the group's lanes
+// split each ring of grid cells, keep private lists pruned by the group's current last distance,
+// and merge them after each ring by rounds of a group-wide (distance, index) arg-min
+// (knn_group_search).  Then the E-step from the supervoxel's moments, candidate j
 // on lane j mod G of the group (lane 0 also takes candidate 4 when G = 4):
 //   L_j = sum_v [-1/2 (3/beta + nu d'Wd) + E ln pi + 1/2 E ln|Lambda|]
 //       = -1/2 (3 n/beta + nu tr(W D)) + n (psi(alpha) - psi(sum alpha) + 1/2 E ln|Lambda|),
@@ -1723,8 +1726,8 @@ __device__ __forceinline__ void ll_issue(const SvRec& R, int t, float* slot, uns
 // candidate ids (stage A, two supervoxels ahead) and its candidates' constants (10
 // doubles each) with its frame's ln(sum alpha) and done flag (stage B, one ahead).
 struct LLRec {
-  SvRec rec;  // the moment pass and the FP64 pass: the SoA spans of the input arrays
-  SvLL ll;    // the moment pass and the FP32 pass: the place in the centred voxel stream
+  SvRec rec;  // the SoA spans of the input arrays
+  SvLL ll;    // the moment pass: the place in the centred voxel stream
   int32_t cand[8];
 };
 struct LLConst {
@@ -1734,8 +1737,7 @@ struct LLConst {
 };
 static_assert(sizeof(LLRec) % 16 == 0 && sizeof(LLConst) % 16 == 0, "look-ahead records stay 16-byte aligned");
 
-// Per-warp shared region: slots, one mbarrier per slot, three stage-A and two stage-B
-// records, and the current supervoxel's FP32 candidate constants.
+// Per-warp shared region: slots, one mbarrier per slot, three stage-A and two stage-B records.
 constexpr int kLLBarOff = kLLStages * kLLSlotFloats * 4;
 constexpr int kLLRecOff = (kLLBarOff + kLLStages * 8 + 15) / 16 * 16;
 constexpr int kLLConstOff = kLLRecOff + 3 * (int)sizeof(LLRec);
@@ -1743,8 +1745,8 @@ constexpr int kLLWarpBytes = (kLLConstOff + 2 * (int)sizeof(LLConst) + 15) / 16 
 constexpr size_t kLLSmemBytes = (size_t)kLLWarpBytes * kLLWarps;
 static_assert((kLLSlotFloats * 4) % 16 == 0 && kLLRecOff % 16 == 0 && kLLConstOff % 16 == 0,
               "slots and records stay 16-byte aligned");
-// the FP32 forms keep kLLBlocks blocks on an SM (228 KB of shared memory, 1 KB reserved per
-// block, the FP32 forms' one static LLShared64); the FP64 form sizes its own grid
+// the moment pass keeps kLLBlocks blocks on an SM (228 KB of shared memory, 1 KB reserved per
+// block, its one static LLShared64); the FP64 form sizes its own grid
 static_assert(kLLBlocks * (kLLSmemBytes + 1024 + sizeof(LLShared64)) <= 233472, "the voxel pass's blocks fit an SM");
 
 // Stage A: the records (SoA spans: kRec; centred-stream place: kLL) and candidate ids
@@ -3005,9 +3007,8 @@ cudaError_t launch_stage_bytes(void* dst, const void* src, size_t bytes, cudaStr
 }
 
 cudaError_t configure_kernels(DevPlan& P, int device) {
-  // every form of the voxel pass: its dynamic shared memory, and the blocks per SM its
-  // persistent grid is sized for -- the fewest of the FP32 forms and the moment pass, and
-  // separately the FP64 form, whose per-warp FP64 constants take more shared memory
+  // the persistent grids: the moment pass, the FP64 log-likelihood (whose per-warp constants take
+  // more shared memory), and the fewest blocks an SM of the FP32 log-likelihood's forms
   const void* forms[2] = {(const void*)k_ll_pass<true>, (const void*)k_ll_pass<false>};
   int sms = 0, per = 1 << 30, per64 = 1 << 30;
   cudaError_t e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
@@ -3061,11 +3062,13 @@ void launch_export(const DevPlan& P, cudaStream_t st) { k_export<<<P.max_gchunks
 // point set, then the queries.
 //   k_sa_bounds  the queries' bounding box and the grid over it (many blocks, the last one
 //                to finish sets the geometry);
-//   k_sa_count   each reference point's cell and its place within the cell;
-//   k_sa_start   each cell's place in the sorted references (cells in any order: the search
-//                orders by (distance, index), so no scan over the cells is needed);
+//   k_sa_count   each reference point's cell and its place within the cell, and the extent of the
+//                cells that hold any;
+//   k_sa_start   each cell's place in the sorted references: the cells of an x-row one after the
+//                other (the searches read a stretch of a row as one range), the rows in any order
+//                (the searches order by (distance, index));
 //   k_sa_fill    the references into their places;
-//   k_sa_query   G lanes per query.
+//   k_sa_query_group, k_sa_query_warp   16 lanes per query, or a warp per 32 (see sa_query).
 // ---------------------------------------------------------------------------
 
 // Scratch of one search over nref points, carved from one buffer (the first kSaClear +
@@ -3719,6 +3722,9 @@ __global__ void __launch_bounds__(128, sa_group_blocks(K)) k_sa_query_group(cons
 // Below this many queries a group of 16 lanes per query, from it on a warp per 32.  Query kernel
 // alone, group / warp: 20,019 queries, K = 10: 48 / 147 us; 60,000: 141 / 196; 200,000 voxels,
 // K = 5: 150 / 82; 1.43 M: 838 / 133.  Groups of 8 and 32: 52 and 47, 150 and 140, 121 and 239.
+// Scattered queries, which the warp form gives to its threads one by one, cost the same on either
+// side of the line: 99,999 of them, 20,000 references, K = 5, 144 us by groups, 100,000 by warps 134
+// (a thread per query without either form 398).
 constexpr int64_t kSaGroupBelow = 100000;
 
 template <int K, bool kMark>

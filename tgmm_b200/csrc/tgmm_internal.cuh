@@ -161,11 +161,11 @@ static_assert(sizeof(SvRec) == 128, "SvRec is eight 16-byte chunks");
 
 // Per-supervoxel record of the log-likelihood pass: where the supervoxel's voxels sit in
 // the plan's centred voxel stream vox4 (one float4 per voxel: x - c0, y - c1, z - c2 in FP32
-// and I, written once per call by the moment pass), its tiles (end-aligned like SvRec's: tile
-// 0 holds r0 voxels, later tiles kVoxTile), its frame and its centroid.
+// and I, written once per call by the moment pass), its frame, its centroid and its extent around
+// that.
 struct SvLL {
   long long v0;
-  int32_t nv, ntiles, frame, frame_nsv;
+  int32_t nv, pad, frame, frame_nsv;
   float c0, c1, c2;
   float h0, h1, h2;  // the largest |x - c| along each axis (the moment pass)
 };
@@ -221,10 +221,10 @@ struct DevPlan {
   // [0] next supervoxel of the voxel pass, [1] warps that left it, [2] next kNN/E-step item of a
   // pass that runs it; zero between launches
   int32_t* work;
-  int32_t ll_blocks;    // resident blocks of the voxel pass's FP32 forms (SMs x blocks per SM)
-  int32_t ll_blocks64;  // the same for its FP64 form
+  int32_t ll_blocks;    // resident blocks of the moment pass (SMs x blocks per SM)
+  int32_t ll_blocks64;  // the same of the FP64 log-likelihood pass
   int32_t ls_blocks;    // blocks of the FP32 log-likelihood pass
-  int32_t knn_group;  // lanes per supervoxel of the kNN/E-step (8, 16 or 32)
+  int32_t knn_group;  // lanes per supervoxel of the kNN/E-step (4, 8, 16 or 32)
   int32_t iter;       // the EM iteration a launch belongs to (1-based; set per launch)
   unsigned long long stage_wait_ns;  // wait limit of a voxel tile copy (default 1 s)
   float4* kpos;  // per Gaussian: the float centre the kNN sees (x, y, z; w = 1 live, 0 dead)
@@ -291,10 +291,7 @@ cudaError_t configure_kernels(DevPlan& P, int device);
 cudaError_t launch_stage_bytes(void* dst, const void* src, size_t bytes, cudaStream_t st);
 void launch_export(const DevPlan& P, cudaStream_t st);
 
-// standalone kNN (tgmm_knn): brute force over refs in shared memory tiles
-cudaError_t knn_bruteforce(const float* query, int64_t nq, const float* ref_xyz, int32_t nref,
-                           const float scale[3], int32_t* ind, cudaStream_t st);
-// grid kNN over a single point set, for tgmm_knn with large nref
+// standalone kNN (tgmm_knn): the grid search over a single point set
 cudaError_t knn_grid_standalone(const float* query, int64_t nq, const float* ref_xyz,
                                 int32_t nref, const float scale[3], int32_t* ind,
                                 cudaStream_t st);
