@@ -28,8 +28,8 @@ extern "C" void run(int warps, long long parts, long long dropped, double v, int
         fixed_acc(ai, ar, v);
         if (p < dropped) di -= i1, dr -= f1;
       }
+      if (carry && parts > 2048) fixed_carry(ai, ar), fixed_carry(di, dr);  // as after a large supervoxel
       ai += di, ar += dr;
-      if (carry) fixed_carry(ai, ar);
       wi += ai, wf += ar;
     }
     if (carry) fixed_carry(wi, wf);

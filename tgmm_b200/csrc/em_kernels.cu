@@ -2235,6 +2235,10 @@ constexpr int kLSRing = TGMM_LS_RING;   // units in flight per warp
 constexpr int kLSUnit = 128;            // voxels per unit, four per lane
 constexpr int kLSFixed = 3;             // supervoxels a warp takes by rule
 constexpr int kLSKept = 1024 / kLSUnit; // units of the reference's kept window
+// A supervoxel of more than a million voxels leaves carried sums, so that a warp's 32 lanes hold
+// fewer than 2^23 parts together: 2^27 voxels of one frame in smaller ones between publications,
+// where the device's memory divided by the warps is some 2^22.
+constexpr int kLSCarryUnits = (1 << 20) / kLSUnit;
 constexpr float kLSZero = -745.13f * kL2E;  // log2 of the smallest positive density
 // Candidates whose terms stay this many bits below the largest one over a whole supervoxel are
 // left out of its sums: at most 4 2^-30 of them, 5e-9 in log2, below the last bit of an FP32 term.
@@ -2545,11 +2549,8 @@ __global__ void __launch_bounds__(kLSWarps * 32, kLSBlocks) k_ll_stream(DevPlan 
   Sh.dr[lane] = 0;
   auto publish = [&]() {
     if (acc_n > 0) {
-      // (what the kept window leaves out was subtracted: ri, rr is a sum of the kept parts alone)
       long long ri = ai + Sh.di[lane];
       unsigned long long rr = ar + Sh.dr[lane];
-      fixed_carry(ai, ar);
-      fixed_carry(ri, rr);
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) {
         ai += __shfl_xor_sync(0xffffffffu, ai, o);
@@ -2782,6 +2783,10 @@ __global__ void __launch_bounds__(kLSWarps * 32, kLSBlocks) k_ll_stream(DevPlan 
         fixed_acc(bi, br, kLn2 * ls_fixup(Sh.cst, P.vox4 + A.ll.v0, nu, kLSUnit - gap, fix));
         Sh.di[lane] += bi;
         Sh.dr[lane] += br;
+      }
+      if (nu > kLSCarryUnits) {
+        fixed_carry(ai, ar);
+        fixed_carry(Sh.di[lane], Sh.dr[lane]);
       }
     } else {
       // its units on their way (all that is) are let land and passed over

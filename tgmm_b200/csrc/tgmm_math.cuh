@@ -6,11 +6,15 @@
 #pragma once
 
 #include <math.h>
+#include <stdint.h>
+#include <string.h>
 
 #ifdef __CUDACC__
 #define TG_HD __host__ __device__ __forceinline__
+#define TG_RARE static __host__ __device__ __noinline__
 #else
 #define TG_HD static inline
+#define TG_RARE static inline
 #endif
 
 // Device code scales by one reciprocal (or reciprocal square root) per shared denominator
@@ -32,10 +36,10 @@ constexpr double kPi = 3.14159265358979323846;
 constexpr double kLnTwoPi = 1.83787706640934548356;  // ln(2*pi)
 
 // Order-free accumulation: a double becomes an (integer, 2^-40 fraction) pair, and pairs add as
-// integers, so a total does not depend on the order of its parts.  A fraction word holds 2^24
-// parts; fixed_carry moves its whole units into the integer and leaves less than one.  Each lane
-// carries before it adds to others' words, so that the limit is 2^24 parts a lane between two
-// publications, and 2^24 publications a frame (at most one a warp of the pass).
+// integers, so a total does not depend on the order of its parts.  A fraction word holds 2^23
+// parts, sums and differences alike; fixed_carry moves its whole units into the integer and leaves
+// less than one.  A warp carries before it adds to its frame's words, so that the limit there is
+// 2^23 publications (at most one a warp of the pass), not parts.
 constexpr double kFracScale = 1099511627776.0;  // 2^40
 TG_HD void fixed_acc(long long& ip, unsigned long long& fp, double v) {
   const double fl = floor(v);
@@ -43,7 +47,7 @@ TG_HD void fixed_acc(long long& ip, unsigned long long& fp, double v) {
   fp += (unsigned long long)((v - fl) * kFracScale);
 }
 TG_HD void fixed_carry(long long& ip, unsigned long long& fp) {
-  ip += (long long)(fp >> 40);
+  ip += (long long)fp >> 40;
   fp &= (1ull << 40) - 1;
 }
 
@@ -328,13 +332,28 @@ TG_HD void regularize_W(double* Wk, double nu, const RegConst& rc) {
   for (int e = 0; e < 6; e++) Wk[e] = W[e] * (double)(rc.scale[ia[e]] * rc.scale[ib[e]]);
 }
 
+// Sign, exponent and upper mantissa bits.
+TG_HD uint32_t hi_word(double v) {
+#if defined(__CUDACC__) && defined(__CUDA_ARCH__)
+  return (uint32_t)__double2hiint(v);
+#else
+  uint64_t b;
+  memcpy(&b, &v, sizeof(b));
+  return (uint32_t)(b >> 32);
+#endif
+}
+// (out of line: the one logarithm's code alone stays in the M-step's)
+TG_RARE double log_weight_parts(double p, double alpha) { return 0.5 * log(p) - 1.5 * kLnTwoPi + log(alpha); }
+
 // ln of a component's weight without the frame's alpha total: ln(alpha) + ln(p)/2 - 3 ln(2 pi)/2 for
 // p = det(nu W).  One logarithm where the product under it is a normal number; an alpha that is
 // not positive has none (NaN, or -inf at 0), and one whose square would underflow keeps its own.
 TG_HD double log_weight(double p, double alpha) {
   const double x = p * (alpha * alpha);
-  if (alpha > 1e-100 && x > 1e-290 && x < 1e290) return 0.5 * log(x) - 1.5 * kLnTwoPi;
-  return 0.5 * log(p) - 1.5 * kLnTwoPi + log(alpha);
+  // 2^-963 <= x < 2^963 and alpha >= 2^-332, by their upper words: the logarithm waits for no
+  // chain of FP64 comparisons (M-step of 12 Gaussians 8.08 us without a test, 8.33 with those)
+  const bool one = hi_word(x) - 0x03c00000u < 0x78600000u && hi_word(alpha) - 0x2b300000u < 0x54c00000u;
+  return one ? 0.5 * log(x) - 1.5 * kLnTwoPi : log_weight_parts(p, alpha);
 }
 
 // E[ln |Lambda|] = 3 ln 2 + ln det W + sum_{i=0..2} psi((nu + 1 - i)/2)
